@@ -235,7 +235,15 @@ int64_t count_steps(double T0, double T1, double dt, double margin, std::vector<
 int cmd::sync(cmd_handle* h) {
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(CMD_ERR_CUDA, std::string("kernel execution: ") + cudaGetErrorString(e));
-    return CMD_OK;
+    return check_fault(h);
+}
+
+// A kernel whose bounded wait gave up sets the handle's fault word; its outputs are not to be used.
+int cmd::check_fault(cmd_handle* h) {
+    volatile int* f = h->hfault.as<int>();
+    if (!f || !*f) return CMD_OK;
+    *f = 0;
+    return fail(CMD_ERR_WATCHDOG, "a wait inside a kernel of this handle gave up: its last results are not valid");
 }
 
 namespace {
@@ -371,6 +379,8 @@ int cmd_create(const cmd_lattice_desc* d, cmd_handle** out) {
     if (cudaGetDevice(&h->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
         rc = fail(CMD_ERR_CUDA, "cudaStreamCreate failed (no CUDA device?)");
+    } else if ((rc = h->hfault.ensure(sizeof(int))) != CMD_OK) {
+        // no page-locked memory for the fault word
     } else if ((rc = noalloc_lookup(&h->noalloc_base)) != CMD_OK) {
         // the device module (with the allocation-free scratch) could not be loaded
     } else if (h->lay.uniform) {
@@ -381,6 +391,7 @@ int cmd_create(const cmd_lattice_desc* d, cmd_handle** out) {
         for (int cs : {2, 4})
             if (rc == CMD_OK) rc = upload_cluster_table(h, cs);
     }
+    if (rc == CMD_OK) *h->hfault.as<int>() = 0;
     if (rc == CMD_OK) rc = h->state.ensure((size_t)h->N * 3 * sizeof(double));
     if (rc == CMD_OK) rc = upload_frames(h, h->frames.data(), h->afm.data());
     if (rc != CMD_OK) {
@@ -399,9 +410,10 @@ int cmd_destroy(cmd_handle* h) {
                       &h->pulses, &h->scratch, &h->dframes, &h->dafm, &h->times, &h->drive, &h->raw,
                       &h->tune_states, &h->tune_obs, &h->gwork, &h->gmeta, &h->gstat, &h->grows, &h->gqueue,
                       &h->awork, &h->ackpt, &h->aseg, &h->amloc, &h->aout, &h->ameta, &h->ain,
-                      &h->sbuf, &h->spart, &h->sgpart, &h->snbase, &h->chunk_states, &h->chunk_rows, &h->cnbr2, &h->cnbr4, &h->cnbr8, &h->cnbr16, &h->cnbr_all, &h->cpush})
+                      &h->sbuf, &h->spart, &h->sgpart, &h->snbase, &h->mid, &h->chunk_states, &h->chunk_rows, &h->cnbr2, &h->cnbr4, &h->cnbr8, &h->cnbr16, &h->cnbr_all, &h->cpush})
         b->release();
     h->hstage.release();
+    h->hfault.release();
     for (cudaStream_t s2 : h->aux_streams) cudaStreamSynchronize(s2);
     for (cudaEvent_t e2 : h->aux_events) cudaEventDestroy(e2);
     for (cudaStream_t s2 : h->aux_streams) cudaStreamDestroy(s2);

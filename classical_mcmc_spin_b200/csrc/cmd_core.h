@@ -73,12 +73,14 @@ struct cmd_handle {
     cmd::DevBuf gwork, gmeta, gstat, grows, gqueue;
     cmd::DevBuf awork, ackpt, aseg, amloc, aout, ameta, ain;
     cmd::DevBuf sbuf, spart, sgpart;  // streamed RK4 / adjoint: stage vectors, tile partials
+    cmd::DevBuf mid;            // states between the slices of a resident batch
     cmd::DevBuf chunk_states, chunk_rows;   // cmd_run_batch: ping-pong states and row buffers of time chunks
     cmd::DevBuf cnbr2, cnbr4, cnbr8, cnbr16;  // partner tables of the 2-, 4-, 8- and 16-CTA cluster kernels
     cmd::DevBuf cnbr_all;       // RK45 on-chip kernels: every slot's partner word per site (built on first use)
     cmd::DevBuf cpush;          // RK45 halo tilings: every site's push words
     int cnbr_all_cs = 0;        // 2 * cluster size (+1 for halo words) cnbr_all / cpush were built for
     cudaStream_t copy_stream = nullptr;  // cmd_run_batch: device-to-host copies of finished chunks
+    cmd::HostBuf hfault;        // one int, page-locked: set by a kernel whose bounded wait gave up
     cmd::HostBuf hstage;        // cmd_run_uneven: page-locked staging of the rows and final states
     std::vector<cudaStream_t> aux_streams;   // concurrent launches of an uneven batch (created on first use)
     // streamed RK4: the stage launches of one chunk of steps captured as a CUDA
@@ -156,9 +158,11 @@ struct Variant {
     bool YREG;
     int TPC;
     int CS;                       // CTAs per trajectory (thread-block cluster), 1 = one CTA
-    bool lean;                    // rk4_lean_kernel (compile-time strides; every atom carries Z bonds)
+    bool flow;                    // rk4_flow_kernel (compile-time strides; every atom carries Z bonds)
     LaunchFn fn;
     const char* name;
+    bool help;                    // rk4_flow_kernel: a helper warp finishes the rows
+    int64_t (*slots)(const cmd_handle*, bool drive);   // trajectories resident at a time, where runs may be sliced
 };
 
 // Streamed adjoint (rk_stream.cuh) for batches too small to fill the GPU with
@@ -227,6 +231,7 @@ inline int global_type(const Layout& L) {
 
 // ---- cmd_api.cu
 int sync(cmd_handle* h);
+int check_fault(cmd_handle* h);
 int caller_atoms(const cmd_handle* h);
 int check_handle(cmd_handle* h, bool need_state);
 int validate_batch(const cmd_handle* h, const cmd_batch_desc* d);
@@ -239,6 +244,9 @@ bool variant_fits(const Variant& v, const Layout& L);
 int default_variant(const Layout& L);
 int pick_variant(const cmd_handle* h);
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches);
+// Sets a.slices / a.slots of a resident batch (a.drive set); the caller provides a.y_mid when a.slices > 1.
+void plan_slices(const cmd_handle* h, const Variant& V, int64_t B, int64_t n_steps, ResidentArgs& a);
+int64_t resident_launches(const ResidentArgs& a, int64_t B);
 int upload_cluster_table(cmd_handle* h, int cs);
 const int* cluster_table(const cmd_handle* h, int cs);
 void variant_shape(const Variant& V, const Layout& L, int64_t* threads, int64_t* smem);

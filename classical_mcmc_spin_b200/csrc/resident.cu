@@ -4,7 +4,7 @@
 // layouts.
 #include "cmd_core.h"
 #include "rk4_cluster.cuh"
-#include "rk4_lean.cuh"
+#include "rk4_flow.cuh"
 
 namespace cmd {
 namespace {
@@ -32,21 +32,50 @@ int launch_one(const cmd_handle* h, const cmd::ResidentArgs& args, const double*
     return CMD_OK;
 }
 
-template <int NAT, int Z, int LZ, int MAXT, int MINB>
-int launch_lean(const cmd_handle* h, const cmd::ResidentArgs& args, const double* d1, const double* d2,
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
+auto flow_kernel(bool stat, bool drive) {
+    return stat ? (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, true, HELP>
+                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, false, HELP>)
+                : (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, true, HELP>
+                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, false, HELP>);
+}
+
+// Trajectories the GPU runs at a time.
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
+int64_t flow_slots(const cmd_handle* h, bool drive) {
+    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h->has_field || h->has_onsite, drive);
+    const int threads = (int)((h->lay.G + 31) / 32 * 32) + (HELP ? 32 : 0);
+    const size_t smem = (size_t)flow_smem_doubles(NAT, MAXT) * sizeof(double);
+    int sms = 0, per = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem) != cudaSuccess)
+        return 0;
+    return (int64_t)sms * per;
+}
+
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
+int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double* d1, const double* d2,
                 int64_t B, cudaStream_t st) {
-    auto kern = cmd::rk4_lean_kernel<NAT, Z, LZ, MAXT, MINB>;
+    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h->has_field || h->has_onsite, args.drive != nullptr);
     const int64_t G = h->lay.G;
-    const int threads = (int)((G + 31) / 32 * 32);
+    const int threads = (int)((G + 31) / 32 * 32) + (HELP ? 32 : 0);
     if (threads > MAXT) return fail(CMD_ERR_UNSUPPORTED, "lattice too large for this kernel variant");
-    const size_t smem = (size_t)cmd::lean_smem_doubles(NAT, MAXT) * sizeof(double);
+    const size_t smem = (size_t)cmd::flow_smem_doubles(NAT, MAXT) * sizeof(double);
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     cmd::Couplings<NAT, Z> cp;
     fill_couplings<NAT, Z>(h, d1, d2, cp);
     cmd::ResidentArgs a = args;
     a.B = B;
-    kern<<<(unsigned)B, threads, smem, st>>>(cp, a);
-    CUDA_TRY(cudaGetLastError());
+    a.fault = h->hfault.as<int>();
+    // items are (slice, trajectory), trajectories fastest: the earlier slice of an item ran in an earlier launch
+    // (slots <= B), so stream order is the only dependence
+    const int64_t items = B * a.slices, per = a.slices > 1 ? a.slots : items;
+    for (int64_t i = 0; i < items; i += per) {
+        a.item0 = i;
+        kern<<<(unsigned)std::min(per, items - i), threads, smem, st>>>(cp, a);
+        CUDA_TRY(cudaGetLastError());
+    }
     return CMD_OK;
 }
 
@@ -90,16 +119,18 @@ int launch_cluster(const cmd_handle* h, const cmd::ResidentArgs& args, const dou
     Variant{NAT, Z, LZ, CPT, MAXT, MINB, YREG, TPC, 1, false, &launch_one<NAT, Z, LZ, CPT, MAXT, MINB, YREG, TPC>, \
             "rk4_resident<" #NAT "," #Z "," #LZ "> cpt=" #CPT " maxt=" #MAXT " minb=" #MINB " yreg=" #YREG \
             " tpc=" #TPC}
-#define CMD_LEAN(NAT, Z, LZ, MAXT, MINB) \
-    Variant{NAT, Z, LZ, 1, MAXT, MINB, true, 1, 1, true, &launch_lean<NAT, Z, LZ, MAXT, MINB>, \
-            "rk4_lean<" #NAT "," #Z "," #LZ "> maxt=" #MAXT " minb=" #MINB}
+#define CMD_FLOW(NAT, Z, LZ, MAXT, MINB, HELP) \
+    Variant{NAT, Z, LZ, 1, MAXT, MINB, true, 1, 1, true, &launch_flow<NAT, Z, LZ, MAXT, MINB, HELP>, \
+            "rk4_flow<" #NAT "," #Z "," #LZ "> maxt=" #MAXT " minb=" #MINB " help=" #HELP, HELP, \
+            &flow_slots<NAT, Z, LZ, MAXT, MINB, HELP>}
 #define CMD_CLUSTER(NAT, Z, LZ, CS, MAXT) \
     Variant{NAT, Z, LZ, 1, MAXT, 1, true, 1, CS, false, &launch_cluster<NAT, Z, LZ, CS, MAXT>, \
             "rk4_cluster<" #NAT "," #Z "," #LZ "> cs=" #CS " maxt=" #MAXT}
 
 const Variant kVariants[] = {
     // 2-atom cells with 3 bonds per site (Kitaev / Heisenberg honeycomb)
-    CMD_LEAN(2, 3, 1, 640, 1),
+    CMD_FLOW(2, 3, 1, 640, 1, true),
+    CMD_FLOW(2, 3, 1, 640, 1, false),
     CMD_VARIANT(2, 3, 1, 1, 640, 1, true, 1),
     CMD_VARIANT(2, 3, 1, 2, 320, 2, false, 1),
     CMD_VARIANT(2, 3, 1, 3, 192, 3, false, 1),
@@ -116,7 +147,7 @@ const Variant kVariants[] = {
     CMD_CLUSTER(2, 3, 1, 2, 640),
     CMD_CLUSTER(2, 3, 1, 4, 640),
     // 4-atom cells with 6 bonds per site (nearest-neighbour pyrochlore)
-    CMD_LEAN(4, 6, 3, 256, 1),
+    CMD_FLOW(4, 6, 3, 256, 1, false),
     CMD_VARIANT(4, 6, 3, 1, 512, 1, true, 1),
     CMD_VARIANT(4, 6, 3, 2, 256, 2, false, 1),
     CMD_VARIANT(4, 6, 3, 2, 512, 1, false, 1),
@@ -159,11 +190,11 @@ const int* cluster_table(const cmd_handle* h, int cs) {
 
 bool variant_fits(const Variant& v, const Layout& L) {
     if (!L.uniform || v.NAT != L.NA || v.Z != L.Z || v.LZ != L.LZ) return false;
-    if (v.lean) {
+    if (v.flow) {
         for (int a = 0; a < L.NA; ++a)
             if (L.zc[a] != L.Z) return false;
-        return (L.G + 31) / 32 * 32 <= v.MAXT &&
-               (size_t)lean_smem_doubles(v.NAT, v.MAXT) * sizeof(double) <= kMaxSmem;
+        return (L.G + 31) / 32 * 32 + (v.help ? 32 : 0) <= v.MAXT &&
+               (size_t)flow_smem_doubles(v.NAT, v.MAXT) * sizeof(double) <= kMaxSmem;
     }
     if (v.CS > 1) {
         const int64_t Gc = cluster_cells(L.G, v.CS);
@@ -198,6 +229,27 @@ int pick_variant(const cmd_handle* h) {
     if (h->variant >= 0 && h->variant < kNumVariants && variant_fits(kVariants[h->variant], h->lay))
         return h->variant;
     return default_variant(h->lay);
+}
+
+// Steps split into slices so that the last, partly filled wave of a batch costs less.  A run of B trajectories on
+// `slots` resident CTAs takes ceil(B / slots) times its steps; cut into K slices, every slots (slice, trajectory)
+// items one launch, ceil(B K / slots) times a K-th of them, plus the start of each launch (kSliceSteps steps' time:
+// launch gap, state, peer masks).  K is the cheapest up to kMaxSlices; one slice unless that saves over 2 %.
+// 768 trajectories of the 24x24 honeycomb on 148 SMs, 2000 steps: 6 waves become 5.2 (figures at rk4_flow.cuh).
+void plan_slices(const cmd_handle* h, const Variant& V, int64_t B, int64_t n_steps, ResidentArgs& a) {
+    constexpr int64_t kSliceSteps = 5, kMaxSlices = 32;
+    a.slices = 1;
+    a.slots = V.slots ? V.slots(h, a.drive != nullptr) : 0;
+    if (a.slots <= 0 || B <= a.slots) return;
+    auto cost = [&](int64_t k) { return (B * k + a.slots - 1) / a.slots * ((n_steps + k - 1) / k + kSliceSteps); };
+    int64_t best = 1;
+    for (int64_t k = 2; k <= kMaxSlices && k <= n_steps; ++k)
+        if (cost(k) < cost(best)) best = k;
+    if (cost(best) * 50 < cost(1) * 49) a.slices = best;
+}
+
+int64_t resident_launches(const ResidentArgs& a, int64_t B) {
+    return a.slices > 1 ? (B * a.slices + a.slots - 1) / a.slots : 1;
 }
 
 // Launches drive-table pre-pass (when driven), the resident kernel and the
@@ -246,6 +298,15 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
         a.drive = h->drive.as<double>();
     }
     if (r.obs && V.NAT != 2 && V.NAT != 4) return fail(CMD_ERR_UNSUPPORTED, "no row finisher for this cell size");
+    plan_slices(h, V, r.B, r.n_steps, a);
+    // one shared initial state that the results overwrite is read by every trajectory's start
+    if (r.y0_stride == 0 && r.y_out && r.y0 >= r.y_out && r.y0 < r.y_out + r.B * h->N * 3) a.slices = 1;
+    if (a.slices > 1) {
+        if (!r.y_out) {
+            if (int rc = h->mid.ensure((size_t)r.B * h->N * 3 * sizeof(double))) return rc;
+        }
+        a.y_mid = r.y_out ? r.y_out : h->mid.as<double>();
+    }
     static const std::vector<double> zeros(3 * 64, 0.0);
     const double* d1 = r.d1 ? r.d1 : zeros.data();
     const double* d2 = r.d2 ? r.d2 : zeros.data();
@@ -260,7 +321,7 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
             ++nl;
         }
         if (int rc2 = V.fn(h, a, d1, d2, r.B, st)) return rc2;
-        ++nl;
+        nl += (int32_t)resident_launches(a, r.B);
         if (r.obs) {
             const int64_t n = r.B * rows;
             const double* fr = r.frames ? r.frames : h->dframes.as<double>();
@@ -278,9 +339,9 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
 }
 
 void variant_shape(const Variant& V, const Layout& L, int64_t* threads, int64_t* smem) {
-    if (V.lean) {
-        *threads = (L.G + 31) / 32 * 32;
-        *smem = (int64_t)lean_smem_doubles(V.NAT, V.MAXT) * (int64_t)sizeof(double);
+    if (V.flow) {
+        *threads = (L.G + 31) / 32 * 32;             // threads with cells
+        *smem = (int64_t)flow_smem_doubles(V.NAT, V.MAXT) * (int64_t)sizeof(double);
     } else if (V.CS > 1) {
         *threads = (cluster_cells(L.G, V.CS) + 31) / 32 * 32;
         *smem = (int64_t)cluster_smem(L.NA, L.G, V.CS);

@@ -70,6 +70,12 @@ struct ResidentArgs {
     long long rows;           // rows per trajectory
     double* traj;             // [B][rows][N*3] or nullptr
     const double* drive;      // [B][n_steps][6] envelope table, or nullptr (no drive)
+    // rk4_flow_kernel: this launch's CTAs run items item0, item0 + 1, ... of slices * B (slice, trajectory) pairs
+    long long item0;
+    long long slices;         // slices of the steps (1: the whole run)
+    long long slots;          // host: items per launch when sliced
+    double* y_mid;            // [B][N*3] states between slices
+    int* fault;               // set when a wait inside the kernel gave up (host-visible)
 };
 
 constexpr int kRedStride = 16;  // doubles per warp in the reduction scratch

@@ -1,0 +1,63 @@
+"""The resident RK4 kernel with waits between warps (rk4_flow.cuh) at the edges of its range.
+
+Cell counts around a warp (16, 32, 33), the largest with a helper warp (608), the smallest without (609), the
+largest a CTA takes (640); and batches larger than the GPU runs at a time, whose steps are cut into slices.
+Tolerances are the path's (test_gpu_parity.py): states 1e-10, rows 1e-12; slices change no arithmetic, so a sliced
+trajectory equals the same one run alone bit for bit.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+R111 = np.ones(3) / np.sqrt(3.0)
+
+
+@pytest.fixture(scope="module")
+def api(native):
+    from classical_mcmc_spin_b200 import gpu_api
+    return gpu_api
+
+
+def _spins(n, seed):
+    from classical_mcmc_spin_b200.states import random_unit_spins
+    return random_unit_spins(n, seed).ravel()
+
+
+@pytest.mark.parametrize("drive", [False, True])
+@pytest.mark.parametrize("dims", [(4, 4), (4, 8), (3, 11), (19, 32), (21, 29), (20, 32)])
+def test_flow_matches_oracle_at_its_edges(api, oracle, dims, drive):
+    from classical_mcmc_spin_b200.lattice import Lattice
+    kw = dict(K=-1.0, Gamma=0.25, Gammap=-0.02, Ka=0.1, Kb=-0.05, Kc=0.02, h=0.1) if dims[0] % 2 else {}
+    lat = Lattice.kitaev(*dims, 1, **kw)
+    o = oracle.OracleLattice.kitaev(*dims, 1, **kw)
+    s0 = _spins(lat.lattice_size, 40 + dims[0])
+    h = lat.to_gpu()
+    assert next(n for _, n, fits in h.variants() if fits).startswith("rk4_flow")     # the default: first that fits
+    if drive:
+        fin = np.tile(R111, 2)
+        api.set_gpu_pulse(h, lat.rotate_pulse(fin, fin), 0.5, 0.5, 0.7, 0.1, 0.6)
+        o.set_pulse(fin, 0.1, fin, 0.6, 0.5, 0.5, 0.7)
+    rows, fin_o = o.md_rk4(s0, 0.0, 0.995, 0.01, 3, gpu_loop=True)
+    api.set_gpu_spins(h, s0)
+    _, obs, _ = api.integrate_gpu(h, 0.0, 0.995, 0.01, 3, "rk4", with_states=False)
+    assert len(obs) == len(rows)
+    assert np.abs(obs - rows[:, 1:11]).max() <= 1e-12
+    assert np.abs(api.get_gpu_spins(h) - fin_o).max() <= 1e-10
+
+
+@pytest.mark.parametrize("dims,B,steps,save", [((24, 24), 301, 97, 3), ((4, 4), 1500, 64, 1), ((19, 32), 151, 40, 50)])
+def test_sliced_batch_equals_single_runs(api, dims, B, steps, save):
+    from classical_mcmc_spin_b200.lattice import Lattice
+    lat = Lattice.kitaev(*dims, 1)
+    h = lat.to_gpu()
+    states = np.stack([_spins(lat.lattice_size, 900 + b) for b in range(B)])
+    fd = lat.rotate_pulse(np.tile(R111, 2), np.tile(R111, 2))
+    t1, t2 = np.linspace(0.0, 0.6, B), np.linspace(0.2, 0.9, B)
+    kw = dict(T0=-0.1, save_interval=save, d1=fd[:6], d2=fd[6:], width=0.3, freq=0.5)
+    obs, fin = api.run_batch(h, states, steps, 0.01, t1=t1, t2=t2, a1=np.full(B, 0.4), a2=np.full(B, 0.3), **kw)
+    for b in (0, 1, B // 2, B - 2, B - 1):
+        o1, f1 = api.run_batch(h, states[b:b + 1], steps, 0.01, t1=t1[b:b + 1], t2=t2[b:b + 1], a1=np.full(1, 0.4),
+                               a2=np.full(1, 0.3), **kw)
+        np.testing.assert_array_equal(obs[b], o1[0])
+        np.testing.assert_array_equal(fin[b], f1[0])
