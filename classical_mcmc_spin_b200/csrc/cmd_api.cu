@@ -477,9 +477,10 @@ int cmd_set_tolerances(cmd_handle* h, double abs_tol, double rel_tol, int64_t ma
 
 namespace {
 
-// Runs `n_steps` RK4 steps of the handle's trajectory on device, saving rows.
+// Runs `n_steps` RK4 (or SSPRK53, where resident_method says so) steps of the handle's trajectory on device, saving
+// rows.
 int run_single(cmd_handle* h, double T0, double dt, int64_t n_steps, int64_t save, double n_sites,
-               bool want_obs, bool want_traj, bool with_pulse) {
+               bool want_obs, bool want_traj, bool with_pulse, int method = CMD_RK4) {
     const int64_t rows = rows_for(n_steps, save);
     if (want_obs)
         if (int rc = h->obs.ensure((size_t)rows * 10 * sizeof(double))) return rc;
@@ -507,7 +508,9 @@ int run_single(cmd_handle* h, double T0, double dt, int64_t n_steps, int64_t sav
     r.d1 = h->fd.data();
     r.d2 = h->fd.data() + 3 * h->NA;
     r.n_sites = n_sites;
-    if (int rc = run_rk4(h, r, h->stream, nullptr)) return rc;
+    r.method = method;
+    if (int rc = method == CMD_RK4 ? run_rk4(h, r, h->stream, nullptr) : run_resident(h, r, h->stream, nullptr))
+        return rc;
     return sync(h);
 }
 
@@ -558,6 +561,8 @@ int run_global_single(cmd_handle* h, int method, double T0, double T1, double dt
     return CMD_OK;
 }
 
+// SSPRK53 on chip (rk4_flow_kernel) where a CTA holds the lattice; the rest runs in global memory.
+bool resident_method(const cmd_handle* h, int method) { return method == CMD_SSPRK53 && flow_variant(h->lay) >= 0; }
 bool resident_fits(const cmd_handle* h) { return pick_variant(h) >= 0; }
 bool rk4_fits(const cmd_handle* h) { return resident_fits(h) || global_type(h->lay) >= 0; }
 
@@ -569,7 +574,8 @@ int cmd_step(cmd_handle* h, double t, double dt, int method) {
     if (!fixed_method(method))
         return fail(CMD_ERR_INVALID_ARG, "cmd_step takes a fixed-step method (any but CMD_RK45)");
     if (!std::isfinite(t) || !std::isfinite(dt)) return fail(CMD_ERR_INVALID_ARG, "non-finite t or dt");
-    if (method == CMD_RK4 && resident_fits(h)) return run_single(h, t, dt, 1, 1, (double)h->N, false, false, true);
+    if ((method == CMD_RK4 && resident_fits(h)) || resident_method(h, method))
+        return run_single(h, t, dt, 1, 1, (double)h->N, false, false, true, method);
     return run_global_single(h, method, t, t + dt, dt, 1, 1, 0, false, nullptr);
 }
 
@@ -605,8 +611,9 @@ int cmd_integrate(cmd_handle* h, double T0, double T1, double dt, int64_t save_i
     const int64_t rows = rows_for(n, save_interval);
     if (rows_out) *rows_out = rows;
     if (max_rows < rows) return fail(CMD_ERR_INVALID_ARG, "max_rows too small");
-    if (method == CMD_RK4 && rk4_fits(h)) {
-        if (int rc = run_single(h, T0, dt, n, save_interval, (double)h->N, obs != nullptr, states != nullptr, true))
+    if ((method == CMD_RK4 && rk4_fits(h)) || resident_method(h, method)) {
+        if (int rc = run_single(h, T0, dt, n, save_interval, (double)h->N, obs != nullptr, states != nullptr, true,
+                                method))
             return rc;
         if (obs) CUDA_TRY(cudaMemcpy(obs, h->obs.p, rows * 10 * sizeof(double), cudaMemcpyDeviceToHost));
     } else {

@@ -131,6 +131,7 @@ struct RunSpec {
     const double* afm = nullptr;      // device [NA]
     double n_sites = 1.0;
     int variant = -1;                 // -1: handle's choice
+    int method = CMD_RK4;             // or CMD_SSPRK53 (one trajectory, lattices flow_variant holds)
 };
 
 // One trajectory of the global-state / on-chip controlled integrators.
@@ -243,6 +244,7 @@ int variant_count();
 bool variant_fits(const Variant& v, const Layout& L);
 int default_variant(const Layout& L);
 int pick_variant(const cmd_handle* h);
+int flow_variant(const Layout& L);
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches);
 // Sets a.slices / a.slots of a resident batch (a.drive set); the caller provides a.y_mid when a.slices > 1.
 void plan_slices(const cmd_handle* h, const Variant& V, int64_t B, int64_t n_steps, ResidentArgs& a);

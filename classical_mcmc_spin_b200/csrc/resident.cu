@@ -32,12 +32,18 @@ int launch_one(const cmd_handle* h, const cmd::ResidentArgs& args, const double*
     return CMD_OK;
 }
 
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP, int NS>
+auto flow_kernel_of(bool stat, bool drive) {
+    return stat ? (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, true, HELP, NS>
+                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, false, HELP, NS>)
+                : (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, true, HELP, NS>
+                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, false, HELP, NS>);
+}
+
 template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
-auto flow_kernel(bool stat, bool drive) {
-    return stat ? (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, true, HELP>
-                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, false, HELP>)
-                : (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, true, HELP>
-                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, false, HELP>);
+auto flow_kernel(bool stat, bool drive, int method = CMD_RK4) {
+    return method == CMD_SSPRK53 ? flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowSSPRK53>(stat, drive)
+                                 : flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowRK4>(stat, drive);
 }
 
 // Trajectories the GPU runs at a time.
@@ -57,7 +63,7 @@ int64_t flow_slots(const cmd_handle* h, bool drive) {
 template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
 int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double* d1, const double* d2,
                 int64_t B, cudaStream_t st) {
-    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h->has_field || h->has_onsite, args.drive != nullptr);
+    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h->has_field || h->has_onsite, args.drive != nullptr, args.method);
     const int64_t G = h->lay.G;
     const int threads = (int)((G + 31) / 32 * 32) + (HELP ? 32 : 0);
     if (threads > MAXT) return fail(CMD_ERR_UNSUPPORTED, "lattice too large for this kernel variant");
@@ -114,6 +120,9 @@ int launch_cluster(const cmd_handle* h, const cmd::ResidentArgs& args, const dou
     CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, cp, a, (int)Gc));
     return CMD_OK;
 }
+
+const StageTimes kSSPRK53Times = {
+    5, {0.0, 0.377268915331368, 0.754537830662736, 0.728985661612188, 0.699226135931670, 0.0, 0.0, 0.0}};
 
 #define CMD_VARIANT(NAT, Z, LZ, CPT, MAXT, MINB, YREG, TPC) \
     Variant{NAT, Z, LZ, CPT, MAXT, MINB, YREG, TPC, 1, false, &launch_one<NAT, Z, LZ, CPT, MAXT, MINB, YREG, TPC>, \
@@ -216,6 +225,13 @@ int default_variant(const Layout& L) {
     return -1;
 }
 
+// The fixed-step methods other than RK4 that run resident (SSPRK53) use the first flow variant that fits.
+int flow_variant(const Layout& L) {
+    for (int i = 0; i < kNumVariants; ++i)
+        if (kVariants[i].flow && variant_fits(kVariants[i], L)) return i;
+    return -1;
+}
+
 int no_instance(const Layout& L) {
     if (!L.uniform) return fail(CMD_ERR_UNSUPPORTED, "lattice layout not supported: " + L.why);
     char buf[200];
@@ -256,12 +272,13 @@ int64_t resident_launches(const ResidentArgs& a, int64_t B) {
 // row-finishing post-pass on `st`.  Asynchronous; returns the launch count.
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches) {
     int32_t nl = 0;
-    const int vi = r.variant >= 0 ? r.variant : pick_variant(h);
+    const int vi = r.method != CMD_RK4 ? flow_variant(h->lay) : (r.variant >= 0 ? r.variant : pick_variant(h));
     if (vi < 0 || !variant_fits(kVariants[vi], h->lay)) return no_instance(h->lay);
     const Variant& V = kVariants[vi];
     const int64_t rows = rows_for(r.n_steps, r.save);
     const int NR = 3 * V.NAT + 1;
     cmd::ResidentArgs a{};
+    a.method = r.method;
     a.G = (int)h->lay.G;
     a.n_steps = r.n_steps;
     a.save_every = r.save;
@@ -293,7 +310,8 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
             t += r.dt;
         }
         if (int rc = h->times.ensure(grid.size() * sizeof(double))) return rc;
-        if (int rc = h->drive.ensure((size_t)r.B * r.n_steps * 6 * sizeof(double))) return rc;
+        const int ne = r.method == CMD_SSPRK53 ? 2 * kSSPRK53Times.n : 6;
+        if (int rc = h->drive.ensure((size_t)r.B * r.n_steps * ne * sizeof(double))) return rc;
         CUDA_TRY(cudaMemcpyAsync(h->times.p, grid.data(), grid.size() * sizeof(double), cudaMemcpyHostToDevice, st));
         a.drive = h->drive.as<double>();
     }
@@ -315,8 +333,12 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
         if (a.drive) {
             const int64_t total = r.B * r.n_steps * 6;
             const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 32);
-            cmd::drive_table_kernel<<<blocks, 256, 0, st>>>(r.pulses, h->times.as<double>(), r.n_steps, r.dt,
-                                                           r.width, r.freq, r.B, h->drive.as<double>());
+            if (r.method == CMD_SSPRK53)
+                cmd::drive_stages_kernel<<<blocks, 256, 0, st>>>(r.pulses, h->times.as<double>(), r.n_steps, r.dt,
+                                                                r.width, r.freq, kSSPRK53Times, h->drive.as<double>());
+            else
+                cmd::drive_table_kernel<<<blocks, 256, 0, st>>>(r.pulses, h->times.as<double>(), r.n_steps, r.dt,
+                                                               r.width, r.freq, r.B, h->drive.as<double>());
             CUDA_TRY(cudaGetLastError());
             ++nl;
         }

@@ -30,7 +30,8 @@
 // instructions).  B200, 1965 MHz: 768 driven trajectories x 2000 steps 32.1 ms (45.5 ms with the barrier and whole
 // waves; 36.9 ms with whole waves); one trajectory 2.80 us per step (3.61); 40 trajectories of 8x8 x 500 steps
 // 0.95 ms (1.35); 200 of the 1024-spin pyrochlore x 800 driven steps 5.27 ms (11.6; atoms interleaved 1.03 us per
-// stage against 1.71).  Polling progress words instead of waiting on mbarriers: 256 instructions, 0.83 us.
+// stage against 1.71); one 24x24 SSPRK53 trajectory x 400 steps, 11 states saved, 1.59 ms (7.05 in global memory,
+// where every RK vector is read and written each stage).  Polling progress words instead of waiting on mbarriers: 256 instructions, 0.83 us.
 #pragma once
 
 #include "rk4_resident.cuh"
@@ -94,7 +95,12 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_
         "DONE:\n\t}" ::"r"(bar), "r"(parity), "r"(dead), "l"(fault) : "memory");
 }
 
-template <int NAT, int Z, int LZ, int MAXT, int MINB, bool STAT, bool DRIVE, bool HELP>
+// Stages per step: classic RK4, or the reference GPU's default method SSPRK(5,3) (integrator.cuh:406-448).
+constexpr int kFlowRK4 = 4, kFlowSSPRK53 = 5;
+
+// NS = stages per step (kFlow*).  Registers hold y, the stage input and one more vector: the RK4 sum, or the second
+// SSPRK(5,3) stage input.
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool STAT, bool DRIVE, bool HELP, int NS>
 __global__ void __launch_bounds__(MAXT, MINB)
 rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ ResidentArgs a) {
     constexpr int NL = Z - LZ;                       // non-local slots per atom
@@ -155,10 +161,11 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
             pb[at][m] = w;
         }
     const double dt = a.dt, half = 0.5 * dt;
-    // envelope factors of the current step: lane e < 6 holds factor e (drive_table_kernel)
-    const bool stager = DRIVE && lane < 6;
-    const double* dtab = stager ? a.drive + b * a.n_steps * 6 + lane : nullptr;
-    double cur_f = stager && n0 < n1 ? dtab[n0 * 6] : 0.0;
+    // envelope factors of the current step: lane e < NE holds factor e (drive_table_kernel, drive_stages_kernel)
+    constexpr int NE = NS == kFlowRK4 ? 6 : 2 * NS;
+    const bool stager = DRIVE && lane < NE;
+    const double* dtab = stager ? a.drive + b * a.n_steps * NE + lane : nullptr;
+    double cur_f = stager && n0 < n1 ? dtab[n0 * NE] : 0.0;
     __syncthreads();
     // a warp is its own peer too, so that every input barrier completes
     if (tid < ncw)
@@ -171,10 +178,10 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     const bool peer = lane < ncw && warp < ncw && (((dep[warp] | (1 << warp)) >> lane) & 1);
     const uint32_t my_in = bar_in + 8 * warp, peer_in = bar_in + 8 * lane;
     // Stage k (counted over the run) waits for phase k / 2 of input barrier k % 2.
-    auto wait_in = [&](int s) { mbar_wait(my_in + 8 * NW * (s & 1), (s >> 1) & 1, dead, a.fault); };
-    auto publish = [&](int s) {                      // the input of stage s is stored
+    auto wait_in = [&](int k) { mbar_wait(my_in + 8 * NW * (k & 1), (k >> 1) & 1, dead, a.fault); };
+    auto publish = [&](int k) {                      // the input of stage k is stored
         __syncwarp();
-        mbar_arrive(peer_in + 8 * NW * (s & 1), peer);
+        mbar_arrive(peer_in + 8 * NW * (k & 1), peer);
     };
     // H = field of the thread's atoms at the stage input S (own atoms) / buffer buf (partners)
     auto field_at = [&](int buf, const double (&S)[NAT][3], double (&H)[NAT][3]) {
@@ -257,6 +264,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     long long save_left = row0 * a.save_every - n0;
     int row = 0;                                     // rows begun here; ring slot row % kFlowRows
     int finisher = 0;                                // warp that finishes the current row (no helper)
+    int k0 = 0;                                      // first stage of the step, mod 4 (0 when a step has 4 stages)
     double part[NV];
     if (HELP && warp == ncw) {
         for (long long n = n0 + save_left; n < n1; n += a.save_every, ++row) {
@@ -270,18 +278,19 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
             save_left = observe ? a.save_every - 1 : save_left - 1;
             const bool driven = DRIVE && __any_sync(0xffffffffu, cur_f != 0.0);   // 0*d adds exactly 0
             double next_f = 0.0;
-            if (stager && step + 1 < n1) next_f = dtab[(step + 1) * 6];
+            if (stager && step + 1 < n1) next_f = dtab[(step + 1) * NE];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const int rb = s & 1;                // buffer read in this stage; the other one is written
-                const int ti = s == 0 ? 0 : (s == 3 ? 2 : 1);
+            for (int s = 0; s < NS; ++s) {
+                const int k = NS == 4 ? s : k0 + s;
+                const int rb = k & 1;                // buffer read in this stage; the other one is written
+                const int ti = NS == kFlowSSPRK53 ? s : (s == 0 ? 0 : (s == 3 ? 2 : 1));
                 if (s == 1 && observe) {
                     mbar_wait(bar_free + 8 * (row % kFlowRows), ((row / kFlowRows) & 1) ^ 1, dead, a.fault);
                     store_partials(part, row % kFlowRows);
                 }
                 const double(&S)[NAT][3] = s == 0 ? y : yc;
                 double H[NAT][3];
-                wait_in(s);
+                wait_in(k);
                 field_at(rb, S, H);
                 if (s == 0 && observe) add_obs(part, S, H);
                 if (driven) {
@@ -295,12 +304,12 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
                             H[at][d] = fma(cp.d2[at][d], f2, H[at][d]);
                         }
                 }
-                double k[NAT][3];
+                double K[NAT][3];
 #pragma unroll
                 for (int at = 0; at < NAT; ++at) {
-                    k[at][0] = H[at][1] * S[at][2] - H[at][2] * S[at][1];
-                    k[at][1] = H[at][2] * S[at][0] - H[at][0] * S[at][2];
-                    k[at][2] = H[at][0] * S[at][1] - H[at][1] * S[at][0];
+                    K[at][0] = H[at][1] * S[at][2] - H[at][2] * S[at][1];
+                    K[at][1] = H[at][2] * S[at][0] - H[at][0] * S[at][2];
+                    K[at][2] = H[at][0] * S[at][1] - H[at][1] * S[at][0];
                 }
                 if (s == 0 && observe && a.traj && own) write_state(a.traj + (b * a.rows + row0 + row) * N3);
                 double* wbuf = smem + (rb ^ 1) * SB;
@@ -308,18 +317,34 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
                 for (int at = 0; at < NAT; ++at)
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        if (s == 3) {
-                            y[at][c] += (dt / 6.0) * (acc[at][c] + k[at][c]);
-                            wbuf[(at * 3 + c) * GS + g] = y[at][c];
+                        if constexpr (NS == kFlowSSPRK53) {          // the reference's 15-digit coefficients
+                            if (s == 0) {
+                                yc[at][c] = 1.0 * y[at][c] + (0.377268915331368 * dt) * K[at][c];
+                            } else if (s == 1) {
+                                yc[at][c] = 1.0 * yc[at][c] + (0.377268915331368 * dt) * K[at][c];
+                                acc[at][c] = yc[at][c];
+                            } else if (s == 2) {
+                                yc[at][c] = 0.355909775063327 * y[at][c] + 0.644090224936674 * acc[at][c] +
+                                            (0.242995220537396 * dt) * K[at][c];
+                            } else if (s == 3) {
+                                yc[at][c] = 0.367933791638137 * y[at][c] + 0.632066208361863 * yc[at][c] +
+                                            (0.238458932846290 * dt) * K[at][c];
+                            } else {
+                                y[at][c] = 0.237593836598569 * acc[at][c] + 0.762406163401431 * yc[at][c] +
+                                           (0.287632146308408 * dt) * K[at][c];
+                            }
+                        } else if (s == 3) {
+                            y[at][c] += (dt / 6.0) * (acc[at][c] + K[at][c]);
                         } else {
-                            acc[at][c] = s == 0 ? k[at][c] : acc[at][c] + 2.0 * k[at][c];
-                            yc[at][c] = 1.0 * y[at][c] + (s == 2 ? dt : half) * k[at][c];
-                            wbuf[(at * 3 + c) * GS + g] = yc[at][c];
+                            acc[at][c] = s == 0 ? K[at][c] : acc[at][c] + 2.0 * K[at][c];
+                            yc[at][c] = 1.0 * y[at][c] + (s == 2 ? dt : half) * K[at][c];
                         }
+                        wbuf[(at * 3 + c) * GS + g] = s == NS - 1 ? y[at][c] : yc[at][c];
                     }
-                publish(s + 1);
+                publish(k + 1);
             }
             cur_f = next_f;
+            if (NS % 4 != 0) k0 = (k0 + NS) & 3;
             if (observe) {
                 if (!HELP) {
                     if (warp == finisher) {
@@ -340,7 +365,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     // Final observation of y(t_end): one more static-field evaluation for E.
     if (warp < ncw) {
         double H[NAT][3];
-        field_at(0, y, H);
+        field_at(NS % 2 == 0 ? 0 : k0 & 1, y, H);
         add_obs(part, y, H);
         if (a.traj && own) write_state(a.traj + (b * a.rows + a.rows - 1) * N3);
         const double r = warp_reduce_many<NV>(part);

@@ -75,6 +75,7 @@ struct ResidentArgs {
     long long slices;         // slices of the steps (1: the whole run)
     long long slots;          // host: items per launch when sliced
     double* y_mid;            // [B][N*3] states between slices
+    int method;               // host: CMD_RK4 or CMD_SSPRK53
     int* fault;               // set when a wait inside the kernel gave up (host-visible)
 };
 
@@ -159,6 +160,26 @@ static __global__ void drive_table_kernel(const Pulse* __restrict__ pulses, cons
         const Pulse p = pulses[b];
         out[e] = (q & 1) ? drive_factor(p.a2, tt - p.t2, width, freq)
                          : drive_factor(p.a1, tt - p.t1, width, freq);
+    }
+}
+
+// Envelope table [n_steps][2 n] of one trajectory: at each step the factors (pulse 1, pulse 2) at the stage times
+// t_n + c[j] dt of a fixed-step method.
+struct StageTimes {
+    int n;
+    double c[8];
+};
+static __global__ void drive_stages_kernel(const Pulse* __restrict__ pulse, const double* __restrict__ times,
+                                           long long n_steps, double dt, double width, double freq,
+                                           const __grid_constant__ StageTimes s, double* __restrict__ out) {
+    const long long total = n_steps * 2 * s.n;
+    const Pulse p = pulse[0];
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        const long long n = e / (2 * s.n);
+        const int q = (int)(e - n * 2 * s.n);
+        const double tt = times[n] + s.c[q >> 1] * dt;
+        out[e] = (q & 1) ? drive_factor(p.a2, tt - p.t2, width, freq) : drive_factor(p.a1, tt - p.t1, width, freq);
     }
 }
 

@@ -61,3 +61,29 @@ def test_sliced_batch_equals_single_runs(api, dims, B, steps, save):
                                a2=np.full(1, 0.3), **kw)
         np.testing.assert_array_equal(obs[b], o1[0])
         np.testing.assert_array_equal(fin[b], f1[0])
+
+
+@pytest.mark.parametrize("drive", [False, True])
+@pytest.mark.parametrize("dims", [(3, 11), (19, 32), (20, 32), (24, 27)])
+def test_ssprk53_matches_oracle_at_its_edges(api, oracle, dims, drive):
+    """SSPRK(5,3) on chip (one warp up to 640 cells) and, for 24x27, in global memory: states to 1e-12 over 40 steps
+    (the bound of test_gpu_methods.py), rows to 1e-13 of the oracle's sums of the returned states."""
+    import fixed_methods as fm
+    from classical_mcmc_spin_b200.lattice import Lattice
+    kw = dict(Ka=0.1, Kb=-0.05, Kc=0.02, h=0.1) if dims[0] % 2 else {}
+    lat = Lattice.kitaev(*dims, 1, **kw)
+    o = oracle.OracleLattice.kitaev(*dims, 1, **kw)
+    s0 = _spins(lat.lattice_size, 70 + dims[0])
+    h = lat.to_gpu()
+    if drive:
+        fin = np.tile(R111, 2)
+        api.set_gpu_pulse(h, lat.rotate_pulse(fin, fin), 0.5, 0.4, 0.9, 0.2, 0.6)
+        o.set_pulse(fin, 0.2, fin, 0.6, 0.5, 0.4, 0.9)
+    api.set_gpu_spins(h, s0)
+    traj, obs, times = api.integrate_gpu(h, 0.0, 0.79, 0.02, 7, "ssprk53")
+    rt, rs = fm.integrate(lambda y, t: o.rhs(y, t), s0, 0.0, 0.79, 0.02, 7, "ssprk53")
+    np.testing.assert_array_equal(times, rt)
+    assert np.abs(np.stack([s for _, s in traj]) - rs).max() <= 1e-12
+    np.testing.assert_array_equal(traj[-1][1], api.get_gpu_spins(h))
+    for r, (_, s) in enumerate(traj):
+        assert np.abs(obs[r, :9] - o.magnetizations(s)).max() <= 1e-13
