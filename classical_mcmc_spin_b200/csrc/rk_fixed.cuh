@@ -51,7 +51,7 @@ __device__ __forceinline__ void lin3(const Ctx& c, double* Z, double a1, const d
 }
 
 template <bool XM, class Ctx>
-__device__ void fixed_step(int mode, const Ctx& c, double* y, double* const* k, double* Ya, double* Yb, double* yn,
+__device__ __forceinline__ void fixed_step(int mode, const Ctx& c, double* y, double* const* k, double* Ya, double* Yb, double* yn,
                            double t, double dt) {
     if (mode == kModeRK4) {                 // integrator.cuh:115-139 arithmetic
         c.sync();
