@@ -62,6 +62,8 @@ int launch_adjoint_cluster(cmd_handle* h, cmd::AdjClusterArgs a, const std::vect
     const int threads = (int)((Gc + 31) / 32 * 32);
     const size_t smem = (size_t)cmd::adj_cluster_smem_doubles(NAT, Gc) * sizeof(double);
     if (threads > MAXT || smem > kMaxSmem) return fail(CMD_ERR_UNSUPPORTED, "lattice too large for this adjoint variant");
+    if (CS > 1)
+        if (int rc = upload_cluster_table(h, CS)) return rc;
     a.nbr = cluster_table(h, CS);
     if (!a.nbr && !h->lay.nbr.empty()) return fail(CMD_ERR_UNSUPPORTED, "no cluster neighbour table for this lattice");
     // Function attributes belong to the current device's context: set on every
@@ -115,7 +117,6 @@ int pick_adjoint_cluster(const cmd_handle* h) {
         if ((Gc + 31) / 32 * 32 > v.MAXT) continue;
         if ((size_t)cmd::adj_cluster_smem_doubles(v.NAT, Gc) * sizeof(double) > kMaxSmem) continue;
         if ((int64_t)v.NAT * 3 * Gc >= (1 << cmd::kClusterRankShift)) continue;
-        if (v.CS > 1 && !cluster_table(h, v.CS)) continue;
         return i;
     }
     return -1;

@@ -43,6 +43,35 @@ bool mat_zero(const double* a) {
     return true;
 }
 
+// Pairs the bonds that leave the cell with the in-cell ones of the same coupling and partner atom (Layout::paired).
+void pair_slots(Layout& L) {
+    const int NL = L.Z - L.LZ;
+    L.paired = false;
+    if (!L.uniform || L.LZ == 0 || NL != L.LZ) return;
+    L.pair.assign((size_t)L.NA * L.LZ, -1);
+    for (int a = 0; a < L.NA; ++a) {
+        if (L.zc[a] != L.Z) return;
+        std::vector<bool> used(NL, false);
+        for (int n = 0; n < L.LZ; ++n)
+            for (int m = 0; m < NL && L.pair[a * L.LZ + n] < 0; ++m) {
+                const int atom = (int)(L.nbr[(size_t)a * NL + m] / (3 * L.G));
+                if (used[m] || atom != (a + 1 + n) % L.NA ||
+                    !mat_equal(&L.J[((size_t)a * L.Z + n) * 9], &L.J[((size_t)a * L.Z + L.LZ + m) * 9]))
+                    continue;
+                used[m] = true;
+                L.pair[a * L.LZ + n] = m;
+            }
+        for (int n = 0; n < L.LZ; ++n)
+            if (L.pair[a * L.LZ + n] < 0) return;
+    }
+    L.nbr_pair.resize(L.nbr.size());
+    for (int64_t g = 0; g < L.G; ++g)
+        for (int a = 0; a < L.NA; ++a)
+            for (int n = 0; n < L.LZ; ++n)
+                L.nbr_pair[((size_t)g * L.NA + a) * NL + n] = L.nbr[((size_t)g * L.NA + a) * NL + L.pair[a * L.LZ + n]];
+    L.paired = true;
+}
+
 // Compile the flat ELL tables into the per-cell layout.  Requirements (every
 // lattice the reference builds from a UnitCell satisfies them): N = NA * G,
 // field/onsite depend on the atom only, and after dropping all-zero coupling
@@ -177,6 +206,7 @@ void analyse_as(const cmd_lattice_desc& d, int NA, Layout& L) {
     };
     if (attempt(true) || attempt(false)) {
         L.uniform = true;
+        pair_slots(L);
         return;
     }
     L.why = "coupling table is not identical in every unit cell";
@@ -388,8 +418,15 @@ int cmd_create(const cmd_lattice_desc* d, cmd_handle** out) {
         if (rc == CMD_OK && !h->lay.nbr.empty() &&
             cudaMemcpy(h->nbr.p, h->lay.nbr.data(), h->lay.nbr.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
             rc = fail(CMD_ERR_CUDA, "neighbour table upload failed");
-        for (int cs : {2, 4})
-            if (rc == CMD_OK) rc = upload_cluster_table(h, cs);
+        if (rc == CMD_OK && h->lay.paired) {
+            rc = h->nbrp.ensure(h->lay.nbr_pair.size() * sizeof(int));
+            if (rc == CMD_OK && cudaMemcpy(h->nbrp.p, h->lay.nbr_pair.data(), h->lay.nbr_pair.size() * sizeof(int),
+                                           cudaMemcpyHostToDevice) != cudaSuccess)
+                rc = fail(CMD_ERR_CUDA, "neighbour table upload failed");
+        }
+        // the table of the default variant's clusters; the others when a variant or the adjoint first needs them
+        const int vi = default_variant(h->lay);
+        if (rc == CMD_OK && vi >= 0) rc = prepare_variant(h, vi);
     }
     if (rc == CMD_OK) *h->hfault.as<int>() = 0;
     if (rc == CMD_OK) rc = h->state.ensure((size_t)h->N * 3 * sizeof(double));
@@ -410,7 +447,7 @@ int cmd_destroy(cmd_handle* h) {
                       &h->pulses, &h->scratch, &h->dframes, &h->dafm, &h->times, &h->drive, &h->raw,
                       &h->tune_states, &h->tune_obs, &h->gwork, &h->gmeta, &h->gstat, &h->grows, &h->gqueue,
                       &h->awork, &h->ackpt, &h->aseg, &h->amloc, &h->aout, &h->ameta, &h->ain,
-                      &h->sbuf, &h->spart, &h->sgpart, &h->snbase, &h->mid, &h->chunk_states, &h->chunk_rows, &h->cnbr2, &h->cnbr4, &h->cnbr8, &h->cnbr16, &h->cnbr_all, &h->cpush})
+                      &h->sbuf, &h->spart, &h->sgpart, &h->snbase, &h->mid, &h->nbrp, &h->nbrt[0], &h->nbrt[1], &h->fctab[2], &h->fctab[4], &h->chunk_states, &h->chunk_rows, &h->cnbr2, &h->cnbr4, &h->cnbr8, &h->cnbr16, &h->cnbr_all, &h->cpush})
         b->release();
     h->hstage.release();
     h->hfault.release();
@@ -1125,6 +1162,8 @@ int cmd_set_variant(cmd_handle* h, int32_t idx) {
     if (idx < -1 || idx >= variant_count()) return fail(CMD_ERR_INVALID_ARG, "variant index out of range");
     if (idx >= 0 && !variant_fits(variant_table()[idx], h->lay))
         return fail(CMD_ERR_UNSUPPORTED, "variant does not fit this lattice");
+    if (idx >= 0)
+        if (int rc = prepare_variant(h, idx)) return rc;
     h->variant = idx;
     return CMD_OK;
 }

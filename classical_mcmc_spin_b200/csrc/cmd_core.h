@@ -50,6 +50,16 @@ struct Layout {
     std::vector<double> J;      // [NA][Z][9]
     std::vector<int> nbr;       // [G][NA][Z-LZ] shared-memory offsets
     std::vector<int> slot_entry;  // [NA][Z] ELL entry at cell 0 each slot came from
+    // every bond that leaves the cell carries the coupling of an in-cell bond to the same atom (a pyrochlore site's up
+    // and down tetrahedra): partner of in-cell slot n is slot LZ + pair[a * LZ + n], and nbr_pair is nbr in that order
+    bool paired = false;
+    std::vector<int> pair, nbr_pair;
+    // tables of rk4_flow_cluster_kernel by cluster size, filled on first use (fits: -1 not computed)
+    struct FlowCluster {
+        int fits = -1;
+        std::vector<int> pw, push, peers;
+    };
+    mutable std::vector<FlowCluster> flow_cluster = std::vector<FlowCluster>(5);
     bool uniform = false;
     std::string why;            // reason when not uniform
     // halo columns of the RK45 cluster partition into cs CTAs (index cs; -1: not
@@ -73,6 +83,9 @@ struct cmd_handle {
     cmd::DevBuf gwork, gmeta, gstat, grows, gqueue;
     cmd::DevBuf awork, ackpt, aseg, amloc, aout, ameta, ain;
     cmd::DevBuf sbuf, spart, sgpart;  // streamed RK4 / adjoint: stage vectors, tile partials
+    cmd::DevBuf nbrp;           // Layout::nbr_pair
+    cmd::DevBuf fctab[5];       // Layout::flow_cluster: pw, push, peers in one buffer, by cluster size
+    cmd::DevBuf nbrt[2];        // partner offsets of the streamed kernels (rk_stream.cuh), unpaired and paired
     cmd::DevBuf mid;            // states between the slices of a resident batch
     cmd::DevBuf chunk_states, chunk_rows;   // cmd_run_batch: ping-pong states and row buffers of time chunks
     cmd::DevBuf cnbr2, cnbr4, cnbr8, cnbr16;  // partner tables of the 2-, 4-, 8- and 16-CTA cluster kernels
@@ -92,10 +105,9 @@ struct cmd_handle {
     // replayed as one graph, the executable graph updated in place per call
     cudaGraphExec_t call_graph[2] = {nullptr, nullptr};
     std::vector<unsigned char> call_sig[2];   // kernels and launch shapes of call_graph[i]
-    // streamed adjoint: one full checkpoint segment (recompute and reverse
-    // sweep) per starting order of the two cotangent buffers, keyed like stream_graph
-    cudaGraphExec_t adj_graph[2] = {nullptr, nullptr};
-    std::vector<unsigned char> adj_graph_key[2];
+    // streamed adjoint: one full checkpoint segment (recompute and reverse sweep), keyed like stream_graph
+    cudaGraphExec_t adj_graph = nullptr;
+    std::vector<unsigned char> adj_graph_key;
     cmd::DevBuf snbase;         // device step base of the replayed chunks
     std::vector<cudaEvent_t> aux_events;
     bool has_state = false;
@@ -243,6 +255,8 @@ const Variant* variant_table();
 int variant_count();
 bool variant_fits(const Variant& v, const Layout& L);
 int default_variant(const Layout& L);
+// Uploads the tables variant vi reads (synchronous, once per handle).
+int prepare_variant(cmd_handle* h, int vi);
 int pick_variant(const cmd_handle* h);
 int flow_variant(const Layout& L);
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches);
@@ -280,6 +294,8 @@ int run_global(cmd_handle* owner, std::vector<GJob>& jobs, int mode, double abs_
 
 // ---- rk45.cu: on-chip controlled Dormand-Prince tilings
 int rk45_variant_count();
+// Halo columns of a cluster partition into cs CTAs of Gc cells (largest of any atom row); see rk45.cu.
+int64_t halo_columns(const Layout& L, int cs, int64_t Gc, std::vector<int>* col);
 const char* rk45_variant_name(int i);
 bool rk45_fits(int i, const Layout& L);
 // The tiling a handle's trajectories use: its tuned pick, else the first that

@@ -5,6 +5,7 @@
 #include "cmd_core.h"
 #include "rk4_cluster.cuh"
 #include "rk4_flow.cuh"
+#include "rk4_flow_cluster.cuh"
 
 namespace cmd {
 namespace {
@@ -32,24 +33,30 @@ int launch_one(const cmd_handle* h, const cmd::ResidentArgs& args, const double*
     return CMD_OK;
 }
 
-template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP, int NS>
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP, int NS, bool PAIR>
 auto flow_kernel_of(bool stat, bool drive) {
-    return stat ? (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, true, HELP, NS>
-                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, false, HELP, NS>)
-                : (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, true, HELP, NS>
-                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, false, HELP, NS>);
+    return stat ? (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, true, HELP, NS, PAIR>
+                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, true, false, HELP, NS, PAIR>)
+                : (drive ? rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, true, HELP, NS, PAIR>
+                         : rk4_flow_kernel<NAT, Z, LZ, MAXT, MINB, false, false, HELP, NS, PAIR>);
 }
 
 template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
-auto flow_kernel(bool stat, bool drive, int method = CMD_RK4) {
-    return method == CMD_SSPRK53 ? flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowSSPRK53>(stat, drive)
-                                 : flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowRK4>(stat, drive);
+auto flow_kernel(const cmd_handle* h, bool drive, int method = CMD_RK4) {
+    const bool stat = h->has_field || h->has_onsite;
+    if constexpr (Z == 2 * LZ) {
+        if (h->lay.paired)
+            return method == CMD_SSPRK53 ? flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowSSPRK53, true>(stat, drive)
+                                         : flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowRK4, true>(stat, drive);
+    }
+    return method == CMD_SSPRK53 ? flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowSSPRK53, false>(stat, drive)
+                                 : flow_kernel_of<NAT, Z, LZ, MAXT, MINB, HELP, kFlowRK4, false>(stat, drive);
 }
 
 // Trajectories the GPU runs at a time.
 template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
 int64_t flow_slots(const cmd_handle* h, bool drive) {
-    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h->has_field || h->has_onsite, drive);
+    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h, drive);
     const int threads = (int)((h->lay.G + 31) / 32 * 32) + (HELP ? 32 : 0);
     const size_t smem = (size_t)flow_smem_doubles(NAT, MAXT) * sizeof(double);
     int sms = 0, per = 0;
@@ -63,7 +70,7 @@ int64_t flow_slots(const cmd_handle* h, bool drive) {
 template <int NAT, int Z, int LZ, int MAXT, int MINB, bool HELP>
 int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double* d1, const double* d2,
                 int64_t B, cudaStream_t st) {
-    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h->has_field || h->has_onsite, args.drive != nullptr, args.method);
+    auto kern = flow_kernel<NAT, Z, LZ, MAXT, MINB, HELP>(h, args.drive != nullptr, args.method);
     const int64_t G = h->lay.G;
     const int threads = (int)((G + 31) / 32 * 32) + (HELP ? 32 : 0);
     if (threads > MAXT) return fail(CMD_ERR_UNSUPPORTED, "lattice too large for this kernel variant");
@@ -74,6 +81,7 @@ int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double
     cmd::ResidentArgs a = args;
     a.B = B;
     a.fault = h->hfault.as<int>();
+    if (h->lay.paired) a.nbr = h->nbrp.as<int>();
     // items are (slice, trajectory), trajectories fastest: the earlier slice of an item ran in an earlier launch
     // (slots <= B), so stream order is the only dependence
     const int64_t items = B * a.slices, per = a.slices > 1 ? a.slots : items;
@@ -81,6 +89,76 @@ int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double
         a.item0 = i;
         kern<<<(unsigned)std::min(per, items - i), threads, smem, st>>>(cp, a);
         CUDA_TRY(cudaGetLastError());
+    }
+    return CMD_OK;
+}
+
+template <int NAT, int Z, int LZ, int CS, int MAXT>
+auto flow_cluster_kernel(const cmd_handle* h, bool drive) {
+    const bool stat = h->has_field || h->has_onsite;
+    auto of = [&](auto pair) {
+        constexpr bool P = decltype(pair)::value != 0;
+        return stat ? (drive ? rk4_flow_cluster_kernel<NAT, Z, LZ, CS, MAXT, true, true, P>
+                             : rk4_flow_cluster_kernel<NAT, Z, LZ, CS, MAXT, true, false, P>)
+                    : (drive ? rk4_flow_cluster_kernel<NAT, Z, LZ, CS, MAXT, false, true, P>
+                             : rk4_flow_cluster_kernel<NAT, Z, LZ, CS, MAXT, false, false, P>);
+    };
+    if constexpr (Z == 2 * LZ) {
+        if (h->lay.paired) return of(AtomTag<1>{});
+    }
+    return of(AtomTag<0>{});
+}
+
+template <int NAT, int CS, int MAXT>
+cudaLaunchConfig_t flow_cluster_config(const cmd_handle* h, int64_t clusters, cudaStream_t st, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * CS));
+    cfg.blockDim = dim3((unsigned)((cluster_cells(h->lay.G, CS) + 31) / 32 * 32 + 32));
+    cfg.dynamicSmemBytes = (size_t)flow_cluster_smem_doubles(NAT, MAXT, CS) * sizeof(double);
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+template <int NAT, int Z, int LZ, int CS, int MAXT>
+int64_t flow_cluster_slots(const cmd_handle* h, bool drive) {
+    auto kern = flow_cluster_kernel<NAT, Z, LZ, CS, MAXT>(h, drive);
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = flow_cluster_config<NAT, CS, MAXT>(h, 1, nullptr, attr);
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess)
+        return 0;
+    return n;
+}
+
+template <int NAT, int Z, int LZ, int CS, int MAXT>
+int launch_flow_cluster(const cmd_handle* h, const cmd::ResidentArgs& args, const double* d1, const double* d2,
+                        int64_t B, cudaStream_t st) {
+    auto kern = flow_cluster_kernel<NAT, Z, LZ, CS, MAXT>(h, args.drive != nullptr);
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    cmd::Couplings<NAT, Z> cp;
+    fill_couplings<NAT, Z>(h, d1, d2, cp);
+    cmd::ResidentArgs a = args;
+    a.B = B;
+    a.fault = h->hfault.as<int>();
+    FlowClusterArgs fc{};
+    const Layout::FlowCluster& t = h->lay.flow_cluster[CS];
+    fc.Gc = (int)cluster_cells(h->lay.G, CS);
+    fc.pw = h->fctab[CS].as<int>();
+    fc.push = fc.pw + t.pw.size();
+    fc.peers = fc.push + t.push.size();
+    const int64_t items = B * a.slices, per = a.slices > 1 ? a.slots : items;   // as launch_flow
+    for (int64_t i = 0; i < items; i += per) {
+        a.item0 = i;
+        cudaLaunchAttribute attr[1];
+        cudaLaunchConfig_t cfg = flow_cluster_config<NAT, CS, MAXT>(h, std::min(per, items - i), st, attr);
+        CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, cp, a, fc));
     }
     return CMD_OK;
 }
@@ -132,6 +210,10 @@ const StageTimes kSSPRK53Times = {
     Variant{NAT, Z, LZ, 1, MAXT, MINB, true, 1, 1, true, &launch_flow<NAT, Z, LZ, MAXT, MINB, HELP>, \
             "rk4_flow<" #NAT "," #Z "," #LZ "> maxt=" #MAXT " minb=" #MINB " help=" #HELP, HELP, \
             &flow_slots<NAT, Z, LZ, MAXT, MINB, HELP>}
+#define CMD_FLOW_CLUSTER(NAT, Z, LZ, CS, MAXT) \
+    Variant{NAT, Z, LZ, 1, MAXT, 1, true, 1, CS, true, &launch_flow_cluster<NAT, Z, LZ, CS, MAXT>, \
+            "rk4_cluster_flow<" #NAT "," #Z "," #LZ "> cs=" #CS " maxt=" #MAXT, true, \
+            &flow_cluster_slots<NAT, Z, LZ, CS, MAXT>}
 #define CMD_CLUSTER(NAT, Z, LZ, CS, MAXT) \
     Variant{NAT, Z, LZ, 1, MAXT, 1, true, 1, CS, false, &launch_cluster<NAT, Z, LZ, CS, MAXT>, \
             "rk4_cluster<" #NAT "," #Z "," #LZ "> cs=" #CS " maxt=" #MAXT}
@@ -153,6 +235,8 @@ const Variant kVariants[] = {
     CMD_VARIANT(2, 3, 1, 1, 640, 1, true, 2),
     CMD_VARIANT(2, 3, 1, 2, 320, 1, false, 2),
     // one trajectory over a cluster of 2 or 4 CTAs (distributed shared memory)
+    CMD_FLOW_CLUSTER(2, 3, 1, 2, 640),
+    CMD_FLOW_CLUSTER(2, 3, 1, 4, 640),
     CMD_CLUSTER(2, 3, 1, 2, 640),
     CMD_CLUSTER(2, 3, 1, 4, 640),
     // 4-atom cells with 6 bonds per site (nearest-neighbour pyrochlore)
@@ -160,6 +244,8 @@ const Variant kVariants[] = {
     CMD_VARIANT(4, 6, 3, 1, 512, 1, true, 1),
     CMD_VARIANT(4, 6, 3, 2, 256, 2, false, 1),
     CMD_VARIANT(4, 6, 3, 2, 512, 1, false, 1),
+    CMD_FLOW_CLUSTER(4, 6, 3, 2, 512),
+    CMD_FLOW_CLUSTER(4, 6, 3, 4, 512),
     CMD_CLUSTER(4, 6, 3, 2, 512),
     CMD_CLUSTER(4, 6, 3, 4, 512),
 };
@@ -186,6 +272,7 @@ int upload_cluster_table(cmd_handle* h, int cs) {
         t[i] = (int)((r << cmd::kClusterRankShift) | ((at * 3 + comp) * Gc + l));
     }
     DevBuf& d = cs == 2 ? h->cnbr2 : h->cnbr4;
+    if (d.p) return CMD_OK;
     if (int rc = d.ensure(std::max<size_t>(t.size(), 1) * sizeof(int))) return rc;
     if (!t.empty() && cudaMemcpy(d.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(CMD_ERR_CUDA, "cluster neighbour table upload failed");
@@ -197,11 +284,82 @@ const int* cluster_table(const cmd_handle* h, int cs) {
     return cs == 1 ? h->nbr.as<int>() : static_cast<const int*>((cs == 2 ? h->cnbr2 : h->cnbr4).p);
 }
 
+// Tables of rk4_flow_cluster_kernel for clusters of cs CTAs of up to maxt - 32 cells: partner offsets (own or halo
+// column), push words, and the peers of every warp.  False when a row needs more halo columns than flow_halo, or a
+// warp has more than kFlowPeers peers.
+bool flow_cluster_plan(const Layout& L, int cs, int maxt) {
+    Layout::FlowCluster& F = L.flow_cluster[cs];
+    if (F.fits >= 0) return F.fits == 1;
+    F.fits = 0;
+    const int NA = L.NA, NL = L.Z - L.LZ;
+    const int64_t G = L.G, Gc = cluster_cells(G, cs), row = maxt + flow_halo(NA), nw = (Gc + 31) / 32;
+    std::vector<int> col;
+    if (NL == 0 || halo_columns(L, cs, Gc, &col) > flow_halo(NA)) return false;
+    const std::vector<int>& nbr = L.paired ? L.nbr_pair : L.nbr;
+    std::vector<int> pw(nbr.size(), 0), push(nbr.size(), -1);
+    std::vector<std::vector<int>> peers((size_t)cs * nw);
+    auto join = [&](int64_t a, int64_t b) {          // warps (rank * nw + warp), both ways
+        for (int k = 0; k < 2; ++k, std::swap(a, b)) {
+            const int w = (int)((b / nw) << 8 | b % nw);
+            std::vector<int>& p = peers[a];
+            if (std::find(p.begin(), p.end(), w) == p.end()) p.push_back(w);
+        }
+    };
+    for (int64_t i = 0; i < (int64_t)peers.size(); ++i) join(i, i);
+    for (size_t i = 0; i < nbr.size(); ++i) {
+        const int64_t site = (int64_t)(i / NL), g = site / NA, r = g / Gc;
+        const int64_t pat = nbr[i] / (3 * G), gp = nbr[i] - pat * 3 * G, rp = gp / Gc;
+        join(r * nw + (g - r * Gc) / 32, rp * nw + (gp - rp * Gc) / 32);
+        if (rp == r) {
+            pw[i] = (int)(pat * 3 * row + gp - r * Gc);
+            continue;
+        }
+        const int64_t slot = pat * 3 * row + maxt + col[((size_t)r * G + gp) * NA + pat];
+        pw[i] = (int)slot;
+        int* to = &push[((size_t)gp * NA + pat) * NL];
+        const int word = (int)(r << kClusterRankShift | slot);
+        int k = 0;
+        while (k < NL && to[k] >= 0 && to[k] != word) ++k;
+        if (k == NL) return false;                   // read by more CTAs than it has bonds
+        to[k] = word;
+    }
+    F.peers.assign(peers.size() * kFlowPeers, -1);
+    for (size_t i = 0; i < peers.size(); ++i) {
+        if (peers[i].size() > (size_t)kFlowPeers) return false;
+        std::copy(peers[i].begin(), peers[i].end(), F.peers.begin() + i * kFlowPeers);
+    }
+    F.pw = std::move(pw);
+    F.push = std::move(push);
+    F.fits = 1;
+    return true;
+}
+
+int prepare_variant(cmd_handle* h, int vi) {
+    const Variant& V = kVariants[vi];
+    if (V.CS == 1) return CMD_OK;
+    if (!V.flow) return upload_cluster_table(h, V.CS);
+    DevBuf& d = h->fctab[V.CS];
+    if (d.p) return CMD_OK;
+    const Layout::FlowCluster& t = h->lay.flow_cluster[V.CS];
+    std::vector<int> all(t.pw);
+    all.insert(all.end(), t.push.begin(), t.push.end());
+    all.insert(all.end(), t.peers.begin(), t.peers.end());
+    if (int rc = d.ensure(all.size() * sizeof(int))) return rc;
+    CUDA_TRY(cudaMemcpy(d.p, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice));
+    return CMD_OK;
+}
+
 bool variant_fits(const Variant& v, const Layout& L) {
     if (!L.uniform || v.NAT != L.NA || v.Z != L.Z || v.LZ != L.LZ) return false;
     if (v.flow) {
         for (int a = 0; a < L.NA; ++a)
             if (L.zc[a] != L.Z) return false;
+        if (v.CS > 1) {
+            const int64_t Gc = cluster_cells(L.G, v.CS);
+            return Gc >= 32 && (Gc + 31) / 32 * 32 + 32 <= v.MAXT &&
+                   (size_t)flow_cluster_smem_doubles(v.NAT, v.MAXT, v.CS) * sizeof(double) <= kMaxSmem &&
+                   flow_cluster_plan(L, v.CS, v.MAXT);
+        }
         return (L.G + 31) / 32 * 32 + (v.help ? 32 : 0) <= v.MAXT &&
                (size_t)flow_smem_doubles(v.NAT, v.MAXT) * sizeof(double) <= kMaxSmem;
     }
@@ -228,7 +386,7 @@ int default_variant(const Layout& L) {
 // The fixed-step methods other than RK4 that run resident (SSPRK53) use the first flow variant that fits.
 int flow_variant(const Layout& L) {
     for (int i = 0; i < kNumVariants; ++i)
-        if (kVariants[i].flow && variant_fits(kVariants[i], L)) return i;
+        if (kVariants[i].flow && kVariants[i].CS == 1 && variant_fits(kVariants[i], L)) return i;
     return -1;
 }
 
@@ -268,13 +426,32 @@ int64_t resident_launches(const ResidentArgs& a, int64_t B) {
     return a.slices > 1 ? (B * a.slices + a.slots - 1) / a.slots : 1;
 }
 
+// The variant of a batch of B trajectories: the handle's, but where nothing was pinned and the default is a
+// one-CTA kernel with a stage barrier, the cluster flow kernel if every trajectory's cluster is resident at once (SMs
+// would idle otherwise), or always where that CTA would hold two 4-atom cells per thread.  B200, per stage and
+// trajectory, one CTA against clusters of 2: honeycomb 27x31 1.63 us on one SM, 0.94 us on two; pyrochlore 500 cells
+// 2.47 / 1.93 us, 864 cells (two per thread, spills) 8.66 / 2.84 us.
+int batch_variant(const cmd_handle* h, int64_t B, bool drive) {
+    const int vi = pick_variant(h);
+    if (vi < 0 || vi == h->variant || kVariants[vi].flow || kVariants[vi].CS > 1) return vi;
+    for (int i = 0; i < kNumVariants; ++i) {
+        const Variant& v = kVariants[i];
+        if (!v.flow || v.CS == 1 || !variant_fits(v, h->lay)) continue;
+        return (kVariants[vi].NAT == 4 && kVariants[vi].CPT > 1) || B <= v.slots(h, drive) ? i : vi;
+    }
+    return vi;
+}
+
 // Launches drive-table pre-pass (when driven), the resident kernel and the
 // row-finishing post-pass on `st`.  Asynchronous; returns the launch count.
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches) {
     int32_t nl = 0;
-    const int vi = r.method != CMD_RK4 ? flow_variant(h->lay) : (r.variant >= 0 ? r.variant : pick_variant(h));
+    const int vi = r.method != CMD_RK4 ? flow_variant(h->lay)
+                   : r.variant >= 0    ? r.variant
+                                       : batch_variant(h, r.B, r.pulses && r.n_steps > 0);
     if (vi < 0 || !variant_fits(kVariants[vi], h->lay)) return no_instance(h->lay);
     const Variant& V = kVariants[vi];
+    if (int rc = prepare_variant(h, vi)) return rc;
     const int64_t rows = rows_for(r.n_steps, r.save);
     const int NR = 3 * V.NAT + 1;
     cmd::ResidentArgs a{};
@@ -361,11 +538,11 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
 }
 
 void variant_shape(const Variant& V, const Layout& L, int64_t* threads, int64_t* smem) {
-    if (V.flow) {
+    if (V.flow && V.CS == 1) {
         *threads = (L.G + 31) / 32 * 32;             // threads with cells
         *smem = (int64_t)flow_smem_doubles(V.NAT, V.MAXT) * (int64_t)sizeof(double);
     } else if (V.CS > 1) {
-        *threads = (cluster_cells(L.G, V.CS) + 31) / 32 * 32;
+        *threads = (cluster_cells(L.G, V.CS) + 31) / 32 * 32;   // threads with cells; own cells' shared memory
         *smem = (int64_t)cluster_smem(L.NA, L.G, V.CS);
     } else {
         *threads = ((L.G + V.CPT - 1) / V.CPT + 31) / 32 * 32;

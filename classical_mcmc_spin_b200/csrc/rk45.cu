@@ -9,23 +9,6 @@
 #include <cstdio>
 
 namespace cmd {
-namespace {
-
-using R45Fn = int (*)(const cmd_handle*, const R45Args&, int64_t, cudaStream_t);
-
-struct R45Variant {
-    int NAT, Z, LZ, APT, CS, MAXT;
-    bool YK;                  // y and K1 in shared memory instead of registers
-    bool HALO;                // partners in other CTAs pushed into halo columns (else read remotely)
-    R45Fn fn;
-    const char* name;
-};
-
-// Cells per CTA and the padded per-atom row of a tiling.
-void r45_shape(const R45Variant& v, int64_t G, int64_t* Gc, int64_t* Gp) {
-    *Gc = (G + v.CS - 1) / v.CS;
-    *Gp = (*Gc + 31) / 32 * 32;
-}
 
 // Halo columns of a cluster partition: for every CTA r, the distinct sites of
 // other CTAs its sites bond to get one column each in the row of their atom,
@@ -55,6 +38,24 @@ int64_t halo_columns(const Layout& L, int cs, int64_t Gc, std::vector<int>* col)
                 }
     }
     return most;
+}
+
+namespace {
+
+using R45Fn = int (*)(const cmd_handle*, const R45Args&, int64_t, cudaStream_t);
+
+struct R45Variant {
+    int NAT, Z, LZ, APT, CS, MAXT;
+    bool YK;                  // y and K1 in shared memory instead of registers
+    bool HALO;                // partners in other CTAs pushed into halo columns (else read remotely)
+    R45Fn fn;
+    const char* name;
+};
+
+// Cells per CTA and the padded per-atom row of a tiling.
+void r45_shape(const R45Variant& v, int64_t G, int64_t* Gc, int64_t* Gp) {
+    *Gc = (G + v.CS - 1) / v.CS;
+    *Gp = (*Gc + 31) / 32 * 32;
 }
 
 // Row length of a tiling's stage buffers: Gp own cells, then the halo columns.

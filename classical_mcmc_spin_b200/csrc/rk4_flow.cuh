@@ -98,9 +98,9 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_
 // Stages per step: classic RK4, or the reference GPU's default method SSPRK(5,3) (integrator.cuh:406-448).
 constexpr int kFlowRK4 = 4, kFlowSSPRK53 = 5;
 
-// NS = stages per step (kFlow*).  Registers hold y, the stage input and one more vector: the RK4 sum, or the second
+// PAIR: the layout's bonds are paired (Layout::paired; a.nbr in that order).  NS = stages per step (kFlow*).  Registers hold y, the stage input and one more vector: the RK4 sum, or the second
 // SSPRK(5,3) stage input.
-template <int NAT, int Z, int LZ, int MAXT, int MINB, bool STAT, bool DRIVE, bool HELP, int NS>
+template <int NAT, int Z, int LZ, int MAXT, int MINB, bool STAT, bool DRIVE, bool HELP, int NS, bool PAIR>
 __global__ void __launch_bounds__(MAXT, MINB)
 rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ ResidentArgs a) {
     constexpr int NL = Z - LZ;                       // non-local slots per atom
@@ -211,11 +211,18 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
 #pragma unroll
             for (int at = 0; at < NAT; ++at) {
                 const int pa = (at + 1 + n) % NAT;
+                // PAIR: slot LZ + n has the same coupling, so J_n (S + P) stands for both bonds
+                double T[3] = {S[pa][0], S[pa][1], S[pa][2]};
+                if constexpr (PAIR) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) T[c] += P[at][n][c];
+                }
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
-                    bond_acc(H[at][d], cp.J[at][n][3 * d], cp.J[at][n][3 * d + 1], cp.J[at][n][3 * d + 2], S[pa][0],
-                             S[pa][1], S[pa][2]);
+                    bond_acc(H[at][d], cp.J[at][n][3 * d], cp.J[at][n][3 * d + 1], cp.J[at][n][3 * d + 2], T[0], T[1],
+                             T[2]);
             }
+        if constexpr (PAIR) return;
 #pragma unroll
         for (int m = 0; m < NL; ++m)
 #pragma unroll

@@ -6,8 +6,8 @@
 // thread advances one site (cell, atom) with rk4_stage_site, the atom uniform
 // per warp, so all SMs work on every trajectory and the kernel boundary is the
 // only barrier between stages (no device-side waits anywhere).  The adjoint
-// uses the same launches for its segment recompute and one vjp_cell launch per
-// stage for the reverse sweep (one cell per thread).
+// uses the same launches for its segment recompute and one stream_vjp_kernel
+// launch per stage for the reverse sweep (one site per thread).
 //
 // Vectors are cell-major SoA per trajectory, v[(atom*3 + c)*G + g], trajectory
 // b at p + b*stride (SVec).  Per stage a cell reads its stage input (own and
@@ -42,7 +42,7 @@ struct StreamArgs {
     int G;                           // cells per trajectory
     int tiles;                       // ceil(G / kStreamTile)
     int B;
-    const int* nbr;
+    const int* nbr;                  // [NAT][Z-LZ][G] partner offsets, cell-minor: a warp's loads are consecutive
     double dt;
     long long n_steps;
     const double* times;             // [n_steps + 1] accumulated t_n
@@ -62,6 +62,7 @@ struct StreamArgs {
     // step base added to every stage launch's step argument, or null (base 0):
     // a replayed launch sequence (CUDA graph) advances it on the device
     const long long* nbase;
+    int b0;                          // first trajectory of the launch (blockIdx.y counts from it)
 };
 
 // Threads of a CTA: NAT groups of kStreamTile/NAT consecutive threads, group
@@ -80,7 +81,8 @@ __device__ __forceinline__ void stream_site(int& at, int& g) {
 // rk4_stage_cell for site (cell g, atom AT) alone.  Every load comes before
 // the first store (acc / Ynext may alias y), so a thread's loads are all in
 // flight together.
-template <int NAT, int Z, int LZ, int AT, int OBS>
+// PAIR: bonds are paired (Layout::paired; nbr in that order), so J_n (S_local + S_far) stands for both.
+template <int NAT, int Z, int LZ, int AT, int OBS, bool PAIR>
 __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, const int* __restrict__ nbr, int G,
                                                int g, double dt, int s, const double* __restrict__ Yin,
                                                const double* y, double* acc, double* Ynext, double f1, double f2,
@@ -106,16 +108,22 @@ __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, cons
 #pragma unroll
     for (int n = 0; n < LZ; ++n) {
         const long long ip = (long long)(((AT + 1 + n) % NAT) * 3) * G + g;
-        const double P0 = Yin[ip], P1 = Yin[ip + G], P2 = Yin[ip + 2 * G];
+        double P0 = Yin[ip], P1 = Yin[ip + G], P2 = Yin[ip + 2 * G];
+        if constexpr (PAIR) {
+            const int p = nbr[(AT * NL + n) * G + g];
+            P0 += Yin[p];
+            P1 += Yin[p + G];
+            P2 += Yin[p + 2 * G];
+        }
 #pragma unroll
         for (int d = 0; d < 3; ++d)
             bond_acc(H[d], cp.J[AT][n][3 * d], cp.J[AT][n][3 * d + 1], cp.J[AT][n][3 * d + 2], P0, P1, P2);
     }
 #pragma unroll
-    for (int m = 0; m < NL; ++m) {
+    for (int m = 0; m < (PAIR ? 0 : NL); ++m) {
         const int n = LZ + m;
         if (n < cp.zc[AT]) {
-            const int p = nbr[((long long)g * NAT + AT) * NL + m];
+            const int p = nbr[(AT * NL + m) * G + g];
             const double P0 = Yin[p], P1 = Yin[p + G], P2 = Yin[p + 2 * G];
 #pragma unroll
             for (int d = 0; d < 3; ++d)
@@ -232,7 +240,7 @@ __device__ __forceinline__ void stream_store_partial(const StreamArgs& a, int b,
 // One RK4 stage s of step n for every (tile, trajectory).  Stage 0 also leaves
 // the observables' partials of Yin (= y_n) and the checkpoint of y_n; the
 // first tile of stage 1 finishes step n's observables.
-template <int NAT, int Z, int LZ>
+template <int NAT, int Z, int LZ, bool PAIR>
 __global__ void __launch_bounds__(kStreamTile, 4)
 stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ StreamArgs a, int s,
                     long long n_arg, SVec Yin, SVec y, SVec acc, SVec Ynext, int with_obs) {
@@ -240,7 +248,7 @@ stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_c
     const long long n = (a.nbase ? *a.nbase : 0) + n_arg;
     __shared__ double red[32 * kRedStride];
     __shared__ double tot[16];
-    const int b = blockIdx.y;
+    const int b = a.b0 + blockIdx.y;
     int at, g;
     stream_site<NAT>(at, g);
     if (s == 1 && with_obs && blockIdx.x == 0) stream_reduce<NAT>(a, b, n, tot);
@@ -255,10 +263,10 @@ stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_c
         with_atom<NAT>(at, [&](auto tag) {
             constexpr int AT = decltype(tag)::value;
             if (s == 0 && with_obs)
-                rk4_stage_site<NAT, Z, LZ, AT, 2>(cp, a.nbr, a.G, g, a.dt, s, yin, y.at(b), acc.at(b), Ynext.at(b),
+                rk4_stage_site<NAT, Z, LZ, AT, 2, PAIR>(cp, a.nbr, a.G, g, a.dt, s, yin, y.at(b), acc.at(b), Ynext.at(b),
                                                   f1, f2, drive, o);
             else
-                rk4_stage_site<NAT, Z, LZ, AT, 0>(cp, a.nbr, a.G, g, a.dt, s, yin, y.at(b), acc.at(b), Ynext.at(b),
+                rk4_stage_site<NAT, Z, LZ, AT, 0, PAIR>(cp, a.nbr, a.G, g, a.dt, s, yin, y.at(b), acc.at(b), Ynext.at(b),
                                                   f1, f2, drive, nullptr);
             if (s == 0 && a.ckpt && n % a.ckpt_every == 0) {
                 double* dst = a.ckpt + ((long long)b * a.n_ckpt + n / a.ckpt_every) * a.V;
@@ -281,12 +289,12 @@ static __global__ void stream_set_base_kernel(long long* nbase, long long v) {
 }
 
 // Observables' partials of y (the state after the last step).
-template <int NAT, int Z, int LZ>
+template <int NAT, int Z, int LZ, bool PAIR>
 __global__ void __launch_bounds__(kStreamTile)
 stream_obs_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ StreamArgs a, SVec y) {
     constexpr int NR = 3 * NAT + 1;
     __shared__ double red[32 * kRedStride];
-    const int b = blockIdx.y;
+    const int b = a.b0 + blockIdx.y;
     int at, g;
     stream_site<NAT>(at, g);
     double o[NR];
@@ -295,7 +303,7 @@ stream_obs_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_con
     if (g < a.G) {
         // a stage-3 pass with no output: only the observables of y are kept
         with_atom<NAT>(at, [&](auto tag) {
-            rk4_stage_site<NAT, Z, LZ, decltype(tag)::value, 2>(cp, a.nbr, a.G, g, a.dt, 3, y.at(b), y.at(b), nullptr,
+            rk4_stage_site<NAT, Z, LZ, decltype(tag)::value, 2, PAIR>(cp, a.nbr, a.G, g, a.dt, 3, y.at(b), y.at(b), nullptr,
                                                                 nullptr, 0.0, 0.0, false, o);
         });
     }
@@ -341,7 +349,7 @@ __global__ void stream_store_kernel(SVec y, int G, double* __restrict__ out) {
 // Adjoint sweep.
 
 struct StreamVjpArgs {
-    int G, tiles;                    // tiles of kStreamTile cells
+    int G, tiles;                    // as StreamArgs
     const int* nbr;
     double dt;
     long long n_steps;
@@ -367,28 +375,169 @@ __global__ void stream_lam_init_kernel(const __grid_constant__ StreamVjpArgs a, 
         for (int c = 0; c < 3; ++c) l[(at * 3 + c) * a.G + g] = 2.0 * (a.mloc[i + c] - a.target[i + c]) / a.n_sites;
 }
 
-// One stage VJP (stage s of step n) for every (tile of kStreamTile cells,
-// trajectory), one cell per thread: mode and buffers as vjp_cell; the tile's
-// parameter cotangents are added to its slot.
-template <int NAT, int Z, int LZ, int NQ>
+// Hbar of the first VJP stage of a segment: hb = Y x (c lam) of every site.
+template <int NAT>
+__global__ void __launch_bounds__(kStreamTile)
+stream_hbar_kernel(int G, double c, SVec Y, SVec lam, SVec hb) {
+    const int b = blockIdx.y;
+    int at, g;
+    stream_site<NAT>(at, g);
+    if (g >= G) return;
+    const long long i = (long long)(at * 3) * G + g;
+    const double *y = Y.at(b) + i, *l = lam.at(b) + i;
+    double* o = hb.at(b) + i;
+    const double y0 = y[0], y1 = y[G], y2 = y[2 * G], v0 = c * l[0], v1 = c * l[G], v2 = c * l[2 * G];
+    o[0] = y1 * v2 - y2 * v1;
+    o[G] = y2 * v0 - y0 * v2;
+    o[2 * G] = y0 * v1 - y1 * v0;
+}
+
+// Coefficients and outputs of one stage VJP: v = ca lam + cb S of this stage; kind 0 (RK stage 3): S = sbar, acc = lam
+// + sbar; 1 (stages 2, 1): S = sbar, acc += sbar; 2 (stage 0): lam = acc + sbar + dl.  Then the next VJP stage's
+// Hbar = Ynext x (ca2 lam + cb2 S), unless Ynext is null.
+struct VjpStage {
+    int s, kind;
+    double ca, cb, ca2, cb2;
+};
+
+// Stage VJP of site (cell g, atom AT).  Y and hb (Hbar = Y x v, formed by the previous VJP stage or
+// stream_hbar_kernel) are read of the partners too, every other vector only at the own site, so lam, S and acc change
+// in place.  Sum over bonds as in vjp_cell; with PAIR (bonds and their parameter derivatives paired) the two partners
+// of a pair are added first.
+template <int NAT, int Z, int LZ, int NQ, int AT, bool PAIR>
+__device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, const ParamDerivs<NAT, Z, NQ>& pd,
+                                                const int* __restrict__ nbr, int G, int g, const VjpStage& st,
+                                                const double* __restrict__ Y, const double* __restrict__ hb,
+                                                double* lam, double* S, double* acc, const double* Ynext, double* hb_out,
+                                                double f1, double f2, bool drive, const double (&dl)[3],
+                                                double (&gq)[NQ]) {
+    constexpr int NL = Z - LZ;
+    const long long i0 = (long long)(AT * 3) * G + g;
+    double Yo[3], ho[3], lo[3], so[3], ao[3], yn[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const long long i = i0 + (long long)c * G;
+        Yo[c] = Y[i];
+        ho[c] = hb[i];
+        lo[c] = lam[i];
+        so[c] = st.kind == 0 ? 0.0 : S[i];
+        ao[c] = st.kind == 0 ? lo[c] : acc[i];
+        yn[c] = Ynext ? Ynext[i] : 0.0;
+    }
+    double H[3], sb[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) H[d] = cp.has_field ? -cp.field[AT][d] : 0.0;
+    if (cp.has_onsite) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            bond_acc(H[d], 2.0 * cp.onsite[AT][3 * d], 2.0 * cp.onsite[AT][3 * d + 1], 2.0 * cp.onsite[AT][3 * d + 2],
+                     Yo[0], Yo[1], Yo[2]);
+            sb[d] += 2.0 * (cp.onsite[AT][d] * ho[0] + cp.onsite[AT][3 + d] * ho[1] + cp.onsite[AT][6 + d] * ho[2]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        double t = -(ho[0] * pd.DB[q][AT][0] + ho[1] * pd.DB[q][AT][1] + ho[2] * pd.DB[q][AT][2]);
+        if (pd.has_DA) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                t += 2.0 * ho[d] * (pd.DA[q][AT][3 * d] * Yo[0] + pd.DA[q][AT][3 * d + 1] * Yo[1] +
+                                    pd.DA[q][AT][3 * d + 2] * Yo[2]);
+        }
+        gq[q] += t;
+    }
+    auto bond = [&](int n, const double (&P)[3], const double (&Q)[3]) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            bond_acc(H[d], cp.J[AT][n][3 * d], cp.J[AT][n][3 * d + 1], cp.J[AT][n][3 * d + 2], P[0], P[1], P[2]);
+            bond_acc(sb[d], cp.J[AT][n][3 * d], cp.J[AT][n][3 * d + 1], cp.J[AT][n][3 * d + 2], Q[0], Q[1], Q[2]);
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            if (!pd.dj_any[q]) continue;             // e.g. a field parameter
+            const double* D = pd.DJ[q][AT][n];
+            gq[q] += Yo[0] * (D[0] * Q[0] + D[1] * Q[1] + D[2] * Q[2]) +
+                     Yo[1] * (D[3] * Q[0] + D[4] * Q[1] + D[5] * Q[2]) +
+                     Yo[2] * (D[6] * Q[0] + D[7] * Q[1] + D[8] * Q[2]);
+        }
+    };
+#pragma unroll
+    for (int n = 0; n < LZ; ++n) {
+        const long long ip = (long long)(((AT + 1 + n) % NAT) * 3) * G + g;
+        double P[3] = {Y[ip], Y[ip + G], Y[ip + 2 * G]}, Q[3] = {hb[ip], hb[ip + G], hb[ip + 2 * G]};
+        if constexpr (PAIR) {
+            const int p = nbr[(AT * NL + n) * G + g];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                P[c] += Y[p + c * G];
+                Q[c] += hb[p + c * G];
+            }
+        }
+        bond(n, P, Q);
+    }
+#pragma unroll
+    for (int m = 0; m < (PAIR ? 0 : NL); ++m)
+        if (LZ + m < cp.zc[AT]) {
+            const int p = nbr[(AT * NL + m) * G + g];
+            const double P[3] = {Y[p], Y[p + G], Y[p + 2 * G]}, Q[3] = {hb[p], hb[p + G], hb[p + 2 * G]};
+            bond(LZ + m, P, Q);
+        }
+    if (drive) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) drive_acc(H[d], cp.d1[AT][d], cp.d2[AT][d], f1, f2);
+    }
+    double v[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        v[c] = st.ca * lo[c];
+        if (st.cb != 0.0) v[c] = v[c] + st.cb * so[c];
+    }
+    sb[0] += v[1] * H[2] - v[2] * H[1];
+    sb[1] += v[2] * H[0] - v[0] * H[2];
+    sb[2] += v[0] * H[1] - v[1] * H[0];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const long long i = i0 + (long long)c * G;
+        if (st.kind == 2) {
+            lo[c] = ao[c] + sb[c] + dl[c];
+            lam[i] = lo[c];
+        } else {
+            S[i] = sb[c];
+            acc[i] = ao[c] + sb[c];
+        }
+        v[c] = st.ca2 * lo[c];
+        if (st.cb2 != 0.0) v[c] = v[c] + st.cb2 * sb[c];
+    }
+    if (Ynext) {
+        hb_out[i0] = yn[1] * v[2] - yn[2] * v[1];
+        hb_out[i0 + G] = yn[2] * v[0] - yn[0] * v[2];
+        hb_out[i0 + 2 * G] = yn[0] * v[1] - yn[1] * v[0];
+    }
+}
+
+// One stage VJP of step n for every (tile, trajectory), one site per thread (atom uniform per warp, so couplings and
+// derivatives are constant-bank operands); the tile's parameter cotangents are added to its slot.
+template <int NAT, int Z, int LZ, int NQ, bool PAIR>
 __global__ void __launch_bounds__(kStreamTile, 3)
 stream_vjp_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ ParamDerivs<NAT, Z, NQ> pd,
-                  const __grid_constant__ StreamVjpArgs a, int s, long long n_arg, SVec Y, SVec lam, SVec Sprev,
-                  double ca, double cb, SVec Sout, SVec acc, SVec lam_out, int mode) {
+                  const __grid_constant__ StreamVjpArgs a, const __grid_constant__ VjpStage st, long long n_arg, SVec Y,
+                  SVec hb, SVec lam, SVec S, SVec acc, SVec Ynext, SVec hb_out) {
+    constexpr int NQV = NQ <= 4 ? 4 : 8;
     const long long n = (a.nbase ? *a.nbase : 0) + n_arg;
     __shared__ double red[32 * kRedStride];
     const int b = blockIdx.y;
-    const int g = blockIdx.x * kStreamTile + threadIdx.x;    // one cell per thread
+    int at, g;
+    stream_site<NAT>(at, g);
     double f1 = 0.0, f2 = 0.0;
     if (a.drive) {
-        const int q = s == 0 ? 0 : (s < 3 ? 2 : 4);
+        const int q = st.s == 0 ? 0 : (st.s < 3 ? 2 : 4);
         const double* d = a.drive + ((long long)b * a.n_steps + n) * 6 + q;
         f1 = d[0];
         f2 = d[1];
     }
     const bool drive = a.drive != nullptr && (f1 != 0.0 || f2 != 0.0);
     double dl[3] = {0.0, 0.0, 0.0};
-    if (mode == 2) {
+    if (st.kind == 2) {
         const long long i = ((long long)b * (a.n_steps + 1) + n) * 3;
 #pragma unroll
         for (int c = 0; c < 3; ++c) dl[c] = 2.0 * (a.mloc[i + c] - a.target[i + c]) / a.n_sites;
@@ -396,26 +545,30 @@ stream_vjp_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_con
     double gq[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) gq[q] = 0.0;
-    if (g < a.G) {
-        vjp_cell<NAT, Z, LZ, NQ>(cp, pd, a.nbr, a.G, g, Y.at(b), lam.at(b), Sprev.at(b), ca, cb, f1, f2, drive,
-                                 Sout.at(b), acc.at(b), lam_out.at(b), mode, dl, gq);
-    }
-    double v[16];
+    if (g < a.G)
+        with_atom<NAT>(at, [&](auto tag) {
+            stream_vjp_site<NAT, Z, LZ, NQ, decltype(tag)::value, PAIR>(
+                cp, pd, a.nbr, a.G, g, st, Y.at(b), hb.at(b), lam.at(b), S.at(b), acc.at(b), Ynext.at(b), hb_out.at(b),
+                f1, f2, drive, dl, gq);
+        });
+    double v[NQV];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = q < NQ ? gq[q] : 0.0;
+    for (int q = 0; q < NQV; ++q) v[q] = q < NQ ? gq[q] : 0.0;
     double t;
-    if (block_sum_par<16>(v, red, NQ, &t)) a.gpart[((long long)b * a.tiles + blockIdx.x) * kPart + threadIdx.x] += t;
+    if (block_sum_par<NQV>(v, red, NQ, &t)) a.gpart[((long long)b * a.tiles + blockIdx.x) * kPart + threadIdx.x] += t;
 }
 
-// grad[b][q] = sum over tiles of the partials (tile order); one CTA per trajectory.
+// grad[b][q] = sum over tiles of the partials, in a fixed order (lane l adds tiles l, l + 32, ..., then a butterfly);
+// one CTA per trajectory, one warp per parameter.
 static __global__ void stream_grad_kernel(const double* __restrict__ gpart, int tiles, int nq, double* __restrict__ out,
                                    long long out_stride) {
-    const int b = blockIdx.x;
-    const int q = threadIdx.x;
+    const int b = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (q >= nq) return;
     double s = 0.0;
-    for (int t = 0; t < tiles; ++t) s += gpart[((long long)b * tiles + t) * kPart + q];
-    out[(long long)b * out_stride + q] = s;
+    for (int t = lane; t < tiles; t += 32) s += gpart[((long long)b * tiles + t) * kPart + q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[(long long)b * out_stride + q] = s;
 }
 
 }  // namespace cmd

@@ -7,26 +7,30 @@
 namespace cmd {
 namespace {
 
-// Steps of the streamed RK4 loop: enqueue(k) launches the four stages of step
-// base + k, base read by the kernels from h->snbase.  With graphs on and at
-// least two chunks of work, one chunk of kChunk steps (4 kChunk stage launches
-// and a base advance) is captured once per distinct set of launch parameters
-// (`key`), kept in the handle and replayed; the remaining steps are launched
-// directly.  The kernels see the same step numbers either way.
+// Steps of the streamed RK4 loop: enqueue(g, k) launches the four stages of step
+// base + k of trajectory group g, base read by the kernels from h->snbase.  A
+// chunk of steps runs group by group, so a group's vectors stay in L2 from stage
+// to stage.  With graphs on and at least two chunks of work, one chunk of
+// kChunk / groups steps (4 kChunk stage launches and a base advance) is captured
+// once per distinct set of launch parameters (`key`), kept in the handle and
+// replayed; the remaining steps are launched directly.  The kernels see the same
+// step numbers either way.
 constexpr int64_t kChunk = 128;
 
 template <class F>
-int run_steps(cmd_handle* h, cudaStream_t st, int64_t S, const std::vector<unsigned char>& key, F&& enqueue,
-              int32_t* nl) {
+int run_steps(cmd_handle* h, cudaStream_t st, int64_t S, int64_t groups, const std::vector<unsigned char>& key,
+              F&& enqueue, int32_t* nl) {
     CUDA_TRY(cudaMemsetAsync(h->snbase.p, 0, sizeof(long long), st));
     int64_t done = 0;
+    const int64_t chunk = std::max<int64_t>(kChunk / groups, 16);
     if (h->graphs && S >= 2 * kChunk) {
         if (!h->stream_graph || h->stream_graph_key != key) {
             release_stream_graph(h);
             cudaGraph_t g = nullptr;
             CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            for (int64_t k = 0; k < kChunk; ++k) enqueue(k);
-            stream_advance_kernel<<<1, 32, 0, st>>>(h->snbase.as<long long>(), kChunk);
+            for (int64_t i = 0; i < groups; ++i)
+                for (int64_t k = 0; k < chunk; ++k) enqueue(i, k);
+            stream_advance_kernel<<<1, 32, 0, st>>>(h->snbase.as<long long>(), chunk);
             const cudaError_t e = cudaStreamEndCapture(st, &g);
             if (e != cudaSuccess || !g) return fail(CMD_ERR_CUDA, std::string("stream capture: ") + cudaGetErrorString(e));
             const cudaError_t e2 = cudaGraphInstantiate(&h->stream_graph, g, 0);
@@ -37,18 +41,49 @@ int run_steps(cmd_handle* h, cudaStream_t st, int64_t S, const std::vector<unsig
             }
             h->stream_graph_key = key;
         }
-        for (; done + kChunk <= S; done += kChunk) {
+        for (; done + chunk <= S; done += chunk) {
             CUDA_TRY(cudaGraphLaunch(h->stream_graph, st));
-            *nl += 4 * (int32_t)kChunk + 1;
+            *nl += (int32_t)(4 * groups * chunk) + 1;
         }
     }
-    for (int64_t k = 0; done + k < S; ++k) {
-        enqueue(k);
-        *nl += 4;
-        if ((k & 1023) == 0) CUDA_TRY(cudaGetLastError());
-    }
-    CUDA_TRY(cudaGetLastError());
+    const int64_t rest = S - done;
+    for (int64_t k0 = 0; k0 < rest; k0 += chunk)
+        for (int64_t i = 0; i < groups; ++i) {
+            const int64_t k1 = std::min(k0 + chunk, rest);
+            for (int64_t k = k0; k < k1; ++k) enqueue(i, k);
+            *nl += (int32_t)(4 * (k1 - k0));
+            CUDA_TRY(cudaGetLastError());
+        }
     return CMD_OK;
+}
+
+// Partner offsets of the streamed kernels, [NAT][Z-LZ][G] (Layout::nbr, or nbr_pair when `pair`); built on first use.
+int stream_table(cmd_handle* h, bool pair) {
+    DevBuf& d = h->nbrt[pair];
+    if (d.p) return CMD_OK;
+    const Layout& L = h->lay;
+    const std::vector<int>& src = pair ? L.nbr_pair : L.nbr;
+    const int NL = L.Z - L.LZ;
+    std::vector<int> t(std::max<size_t>(src.size(), 1));
+    for (int64_t g = 0; g < L.G; ++g)
+        for (int a = 0; a < L.NA; ++a)
+            for (int m = 0; m < NL; ++m)
+                t[((size_t)a * NL + m) * L.G + g] = src[((size_t)g * L.NA + a) * NL + m];
+    if (int rc = d.ensure(t.size() * sizeof(int))) return rc;
+    CUDA_TRY(cudaMemcpy(d.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice));
+    return CMD_OK;
+}
+
+// Trajectories per group of a streamed run with `vectors` vectors of V doubles each: as many as keep the group's
+// vectors within kL2Share of L2 (measured on the 65536-spin pyrochlore, 32 trajectories: see rk_stream.cuh), in
+// groups of equal size.
+int64_t stream_group(const cmd_handle* h, int64_t B, int64_t V, int vectors) {
+    int l2 = 0;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device) != cudaSuccess || l2 <= 0) return B;
+    constexpr double kL2Share = 0.6;
+    const int64_t fit = std::max<int64_t>(1, (int64_t)(kL2Share * l2 / ((double)vectors * V * sizeof(double))));
+    const int64_t groups = (B + fit - 1) / fit;
+    return (B + groups - 1) / groups;
 }
 
 template <class T>
@@ -62,7 +97,7 @@ void key_add(std::vector<unsigned char>& k, const T& v) {
 // per stage over (cell tile, trajectory); same RunSpec contract and outputs as
 // run_resident.
 
-template <int NAT, int Z, int LZ>
+template <int NAT, int Z, int LZ, bool PAIR>
 int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches) {
     constexpr int NR = 3 * NAT + 1;
     int32_t nl = 0;
@@ -81,7 +116,8 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
     a.G = G;
     a.tiles = tiles;
     a.B = (int)B;
-    a.nbr = h->nbr.as<int>();
+    if (int rc = stream_table(h, PAIR)) return rc;
+    a.nbr = h->nbrt[PAIR].as<int>();
     a.dt = r.dt;
     a.n_steps = r.n_steps;
     a.part = h->spart.as<double>();
@@ -136,10 +172,10 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
     if (r.traj) {                                    // states saved between steps: direct launches
         for (int64_t n = 0; n < r.n_steps; ++n) {
             if (n % r.save == 0) save_traj(n / r.save);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 0, n, y, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 1, n, Ya, y, acc, Yb, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 2, n, Yb, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 3, n, Ya, y, acc, y, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 0, n, y, y, acc, Ya, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 1, n, Ya, y, acc, Yb, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 2, n, Yb, y, acc, Ya, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 3, n, Ya, y, acc, y, with_obs);
             nl += 4;
             if ((n & 1023) == 0) CUDA_TRY(cudaGetLastError());
         }
@@ -158,18 +194,23 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
         key_add(key, Yb);
         key_add(key, with_obs);
         key_add(key, grid);
-        auto enqueue = [&](int64_t k) {
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 0, k, y, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 1, k, Ya, y, acc, Yb, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 2, k, Yb, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 3, k, Ya, y, acc, y, with_obs);
+        const int64_t per = stream_group(h, B, V, 4), groups = (B + per - 1) / per;
+        key_add(key, per);
+        auto enqueue = [&](int64_t i, int64_t k) {
+            cmd::StreamArgs ag = a;
+            ag.b0 = (int)(i * per);
+            const dim3 gg(tiles, (unsigned)std::min(per, B - i * per));
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 0, k, y, y, acc, Ya, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 1, k, Ya, y, acc, Yb, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 2, k, Yb, y, acc, Ya, with_obs);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 3, k, Ya, y, acc, y, with_obs);
         };
-        if (int rc = run_steps(h, st, r.n_steps, key, enqueue, &nl)) return rc;
+        if (int rc = run_steps(h, st, r.n_steps, groups, key, enqueue, &nl)) return rc;
         a.nbase = nullptr;                           // the final observation below uses absolute steps
     }
     if (r.traj) save_traj(rows - 1);
     if (r.obs) {
-        cmd::stream_obs_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, y);
+        cmd::stream_obs_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, y);
         cmd::stream_reduce_kernel<NAT><<<(unsigned)B, cmd::kStreamTile, 0, st>>>(a, r.n_steps);
         CUDA_TRY(cudaGetLastError());
         nl += 2;
@@ -190,7 +231,7 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
     return CMD_OK;
 }
 
-template <int NAT, int Z, int LZ, int NQ>
+template <int NAT, int Z, int LZ, int NQ, bool PAIR>
 int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<double>& DJ, const std::vector<double>& DB,
                    const std::vector<double>& DA, bool has_DA) {
     cudaStream_t st = h->stream;
@@ -199,8 +240,7 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
     const int64_t V = (int64_t)NAT * 3 * G, B = j.B, S = j.S, C = j.C, K = j.K;
     if (int rc = h->sbuf.ensure((size_t)5 * B * V * sizeof(double))) return rc;
     if (int rc = h->spart.ensure(((size_t)B * tiles * cmd::kPart + B) * sizeof(double))) return rc;
-    const int vtiles = (G + cmd::kStreamTile - 1) / cmd::kStreamTile;     // VJP: one cell per thread
-    if (int rc = h->sgpart.ensure((size_t)B * vtiles * cmd::kPart * sizeof(double))) return rc;
+    if (int rc = h->sgpart.ensure((size_t)B * tiles * cmd::kPart * sizeof(double))) return rc;
     double* base = h->sbuf.as<double>();
     double* d_loss = h->spart.as<double>() + (size_t)B * tiles * cmd::kPart;
     const bool driven = h->amp != 0.0;
@@ -221,7 +261,8 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
     a.G = G;
     a.tiles = tiles;
     a.B = (int)B;
-    a.nbr = h->nbr.as<int>();
+    if (int rc = stream_table(h, PAIR)) return rc;
+    a.nbr = h->nbrt[PAIR].as<int>();
     a.dt = j.dt;
     a.n_steps = S;
     a.times = j.times;
@@ -256,15 +297,20 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
         key_add(key, Ya);
         key_add(key, Yb);
         key_add(key, grid);
-        auto enqueue = [&](int64_t k) {
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, af, 0, k, y, y, acc, Ya, 1);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, af, 1, k, Ya, y, acc, Yb, 1);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, af, 2, k, Yb, y, acc, Ya, 1);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, af, 3, k, Ya, y, acc, y, 1);
+        const int64_t per = stream_group(h, B, V, 4), groups = (B + per - 1) / per;
+        key_add(key, per);
+        auto enqueue = [&](int64_t i, int64_t k) {
+            cmd::StreamArgs ag = af;
+            ag.b0 = (int)(i * per);
+            const dim3 gg(tiles, (unsigned)std::min(per, B - i * per));
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 0, k, y, y, acc, Ya, 1);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 1, k, Ya, y, acc, Yb, 1);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 2, k, Yb, y, acc, Ya, 1);
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 3, k, Ya, y, acc, y, 1);
         };
         int32_t nl = 0;
-        if (int rc = run_steps(h, st, S, key, enqueue, &nl)) return rc;
-        cmd::stream_obs_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, y);
+        if (int rc = run_steps(h, st, S, groups, key, enqueue, &nl)) return rc;
+        cmd::stream_obs_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, y);
         cmd::stream_reduce_kernel<NAT><<<(unsigned)B, cmd::kStreamTile, 0, st>>>(a, S);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpy2DAsync(j.out, (1 + kAdjParams) * sizeof(double), d_loss, sizeof(double), sizeof(double),
@@ -281,9 +327,13 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
             std::memcpy(pd.DA[q][at], &DA[((size_t)q * NAT + at) * 9], 9 * sizeof(double));
         }
     pd.has_DA = has_DA;
+    for (int q = 0; q < NQ; ++q)
+        for (int at = 0; at < NAT; ++at)
+            for (int sl = 0; sl < Z; ++sl)
+                for (int e = 0; e < 9; ++e) pd.dj_any[q] |= pd.DJ[q][at][sl][e] != 0.0;
     cmd::StreamVjpArgs v{};
     v.G = G;
-    v.tiles = vtiles;
+    v.tiles = tiles;
     v.nbr = a.nbr;
     v.dt = j.dt;
     v.n_steps = S;
@@ -294,57 +344,52 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
     v.gpart = h->sgpart.as<double>();
     cmd::StreamArgs ar = a;              // recompute: no observables, no checkpoints
     ar.ckpt = nullptr;
-    CUDA_TRY(cudaMemsetAsync(v.gpart, 0, (size_t)B * vtiles * cmd::kPart * sizeof(double), st));
-    const dim3 vgrid(vtiles, (unsigned)B);
-    cmd::SVec lam{base, V}, lam2{base + B * V, V};
-    const cmd::SVec acc{base + 2 * B * V, V}, Sa{base + 3 * B * V, V}, Sb{base + 4 * B * V, V};
+    CUDA_TRY(cudaMemsetAsync(v.gpart, 0, (size_t)B * tiles * cmd::kPart * sizeof(double), st));
+    const cmd::SVec lam{base, V}, acc{base + B * V, V}, Sv{base + 2 * B * V, V};
+    const cmd::SVec hb[2] = {{base + 3 * B * V, V}, {base + 4 * B * V, V}};
     cmd::stream_lam_init_kernel<NAT><<<gridc, 256, 0, st>>>(v, lam);
     double* seg = h->aseg.as<double>();
     auto slot = [&](int64_t jj, int q) { return cmd::SVec{seg + (jj * 4 + q) * V, C * 4 * V}; };
     const double dt = j.dt;
     // One checkpoint segment of len steps: the recompute that stores every
     // stage input, then the reverse sweep; kernel step arguments are nb + jj.
-    // The cotangent buffers l / l2 swap once per step.
-    auto segment = [&](int64_t len, int64_t nb, const cmd::StreamArgs& sa, const cmd::StreamVjpArgs& sv,
-                       cmd::SVec& l, cmd::SVec& l2) {
+    auto segment = [&](int64_t len, int64_t nb, const cmd::StreamArgs& sa, const cmd::StreamVjpArgs& sv) {
         for (int64_t jj = 0; jj < len; ++jj) {
             const int64_t n = nb + jj;
             const cmd::SVec y = slot(jj, 0);
             const cmd::SVec last = jj + 1 < len ? slot(jj + 1, 0) : none;
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 0, n, y, y, acc,
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 0, n, y, y, acc,
                                                                                    slot(jj, 1), 0);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 1, n, slot(jj, 1), y, acc,
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 1, n, slot(jj, 1), y, acc,
                                                                                    slot(jj, 2), 0);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 2, n, slot(jj, 2), y, acc,
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 2, n, slot(jj, 2), y, acc,
                                                                                    slot(jj, 3), 0);
-            cmd::stream_stage_kernel<NAT, Z, LZ><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 3, n, slot(jj, 3), y, acc,
+            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 3, n, slot(jj, 3), y, acc,
                                                                                    last, 0);
         }
+        cmd::stream_hbar_kernel<NAT><<<grid, cmd::kStreamTile, 0, st>>>(G, dt / 6.0, slot(len - 1, 3), lam, hb[0]);
         for (int64_t jj = len - 1; jj >= 0; --jj) {
             const int64_t n = nb + jj;
-            auto vjp = cmd::stream_vjp_kernel<NAT, Z, LZ, NQ>;
-            vjp<<<vgrid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, 3, n, slot(jj, 3), l, none, dt / 6.0, 0.0, Sa, acc,
-                                                   none, 0);
-            vjp<<<vgrid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, 2, n, slot(jj, 2), l, Sa, dt / 3.0, dt, Sb, acc,
-                                                   none, 1);
-            vjp<<<vgrid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, 1, n, slot(jj, 1), l, Sb, dt / 3.0, 0.5 * dt, Sa,
-                                                   acc, none, 1);
-            vjp<<<vgrid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, 0, n, slot(jj, 0), l, Sa, dt / 6.0, 0.5 * dt, none,
-                                                   acc, l2, 2);
-            std::swap(l, l2);
+            auto vjp = cmd::stream_vjp_kernel<NAT, Z, LZ, NQ, PAIR>;
+            const double c6 = dt / 6.0, c3 = dt / 3.0;
+            const cmd::VjpStage s3{3, 0, c6, 0.0, c3, dt}, s2{2, 1, c3, dt, c3, 0.5 * dt};
+            const cmd::VjpStage s1{1, 1, c3, 0.5 * dt, c6, 0.5 * dt}, s0{0, 2, c6, 0.5 * dt, c6, 0.0};
+            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s3, n, slot(jj, 3), hb[0], lam, Sv, acc, slot(jj, 2), hb[1]);
+            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s2, n, slot(jj, 2), hb[1], lam, Sv, acc, slot(jj, 1), hb[0]);
+            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s1, n, slot(jj, 1), hb[0], lam, Sv, acc, slot(jj, 0), hb[1]);
+            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s0, n, slot(jj, 0), hb[1], lam, Sv, acc,
+                                                  jj > 0 ? slot(jj - 1, 3) : none, hb[0]);
         }
     };
     // Full-length segments replay a captured graph of the segment with the
     // kernels' steps relative to the device step base (set to the segment's
-    // first step before each replay); one graph per order of the cotangent
-    // buffers at the segment's start.  The partial segment (processed first)
+    // first step before each replay).  The partial segment (processed first)
     // and, with graphs off, every segment launch directly.
     if (int rc = h->snbase.ensure(sizeof(long long))) return rc;
     cmd::StreamArgs ar_rel = ar;
     ar_rel.nbase = h->snbase.as<long long>();
     cmd::StreamVjpArgs v_rel = v;
     v_rel.nbase = h->snbase.as<long long>();
-    const double* lam_start = lam.p;
     for (int64_t sg = K - 1; sg >= 0; --sg) {
         const int64_t n0 = sg * C, n1 = std::min(n0 + C, S);
         CUDA_TRY(cudaMemcpy2DAsync(seg, (size_t)C * 4 * V * sizeof(double), h->ackpt.as<double>() + sg * V,
@@ -352,42 +397,35 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
                                    cudaMemcpyDeviceToDevice, st));
         const int64_t len = n1 - n0;
         if (!h->graphs || len != C || K < 3) {
-            segment(len, n0, ar, v, lam, lam2);
+            segment(len, n0, ar, v);
             CUDA_TRY(cudaGetLastError());
             continue;
         }
-        const int par = lam.p == lam_start ? 0 : 1;
         std::vector<unsigned char> key;
         key_add(key, 3);                             // adjoint segment of this NAT/Z/LZ/NQ
-        key_add(key, NAT * 1000 + Z * 100 + LZ * 10 + NQ);
+        key_add(key, NAT * 10000 + Z * 1000 + LZ * 100 + NQ * 10 + PAIR);
         key_add(key, cp);
         key_add(key, pd);
         key_add(key, ar_rel);
         key_add(key, v_rel);
         key_add(key, lam);
-        key_add(key, lam2);
-        key_add(key, acc);
-        key_add(key, Sa);
-        key_add(key, Sb);
         key_add(key, seg);
         key_add(key, C);
         key_add(key, grid);
-        key_add(key, vgrid);
         key_add(key, dt);
         cmd::stream_set_base_kernel<<<1, 32, 0, st>>>(h->snbase.as<long long>(), n0);
         CUDA_TRY(cudaGetLastError());
-        cudaGraphExec_t& ex = h->adj_graph[par];
-        if (!ex || h->adj_graph_key[par] != key) {
+        cudaGraphExec_t& ex = h->adj_graph;
+        if (!ex || h->adj_graph_key != key) {
             if (ex) {
                 cudaStreamSynchronize(st);
                 cudaGraphExecDestroy(ex);
                 ex = nullptr;
             }
-            h->adj_graph_key[par].clear();
-            cmd::SVec l = lam, l2 = lam2;
+            h->adj_graph_key.clear();
             cudaGraph_t g = nullptr;
             CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            segment(len, 0, ar_rel, v_rel, l, l2);
+            segment(len, 0, ar_rel, v_rel);
             const cudaError_t e = cudaStreamEndCapture(st, &g);
             if (e != cudaSuccess || !g) {
                 if (g) cudaGraphDestroy(g);
@@ -399,12 +437,11 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
                 ex = nullptr;
                 return fail(CMD_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e2));
             }
-            h->adj_graph_key[par] = key;
+            h->adj_graph_key = key;
         }
         CUDA_TRY(cudaGraphLaunch(ex, st));
-        if (len & 1) std::swap(lam, lam2);
     }
-    cmd::stream_grad_kernel<<<(unsigned)B, 32, 0, st>>>(v.gpart, vtiles, NQ, j.out + 1, 1 + kAdjParams);
+    cmd::stream_grad_kernel<<<(unsigned)B, 32 * NQ, 0, st>>>(v.gpart, tiles, NQ, j.out + 1, 1 + kAdjParams);
     CUDA_TRY(cudaGetLastError());
     return CMD_OK;
 }
@@ -421,10 +458,10 @@ void release_stream_graph(cmd_handle* h) {
         if (h->call_graph[i]) cudaGraphExecDestroy(h->call_graph[i]);
         h->call_graph[i] = nullptr;
         h->call_sig[i].clear();
-        if (h->adj_graph[i]) cudaGraphExecDestroy(h->adj_graph[i]);
-        h->adj_graph[i] = nullptr;
-        h->adj_graph_key[i].clear();
     }
+    if (h->adj_graph) cudaGraphExecDestroy(h->adj_graph);
+    h->adj_graph = nullptr;
+    h->adj_graph_key.clear();
 }
 
 namespace {
@@ -513,8 +550,10 @@ int graph_call(cmd_handle* h, int slot, cudaStream_t st, const std::function<int
 
 int run_streamed(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches) {
     switch (global_type(h->lay)) {
-        case 0: return stream_forward<2, 3, 1>(h, r, st, launches);
-        case 1: return stream_forward<4, 6, 3>(h, r, st, launches);
+        case 0: return stream_forward<2, 3, 1, false>(h, r, st, launches);
+        case 1:
+            return h->lay.paired ? stream_forward<4, 6, 3, true>(h, r, st, launches)
+                                 : stream_forward<4, 6, 3, false>(h, r, st, launches);
         default: return no_instance(h->lay);
     }
 }
@@ -523,12 +562,25 @@ int run_stream_adjoint(cmd_handle* h, const StreamAdjJob& j, int n_params, const
                        const std::vector<double>& DB, const std::vector<double>& DA, bool has_DA) {
     const int ty = global_type(h->lay);
     if (ty < 0) return no_instance(h->lay);
+    // paired bonds: their parameter derivatives must be too
+    const Layout& L = h->lay;
+    bool pair = L.paired;
+    const int nq = n_params <= 4 ? 4 : 5;
+    for (int q = 0; q < nq && pair; ++q)
+        for (int at = 0; at < L.NA && pair; ++at)
+            for (int n = 0; n < L.LZ && pair; ++n) {
+                const double* D = &DJ[((size_t)q * L.NA + at) * L.Z * 9];
+                pair = std::memcmp(D + 9 * n, D + 9 * (L.LZ + L.pair[at * L.LZ + n]), 9 * sizeof(double)) == 0;
+            }
     // the VJP carries as many parameter cotangents as requested (4 or 5)
-    if (n_params <= 4)
-        return ty == 0 ? stream_adjoint<2, 3, 1, 4>(h, j, DJ, DB, DA, has_DA)
-                       : stream_adjoint<4, 6, 3, 4>(h, j, DJ, DB, DA, has_DA);
-    return ty == 0 ? stream_adjoint<2, 3, 1, 5>(h, j, DJ, DB, DA, has_DA)
-                   : stream_adjoint<4, 6, 3, 5>(h, j, DJ, DB, DA, has_DA);
+    if (ty == 0)
+        return nq == 4 ? stream_adjoint<2, 3, 1, 4, false>(h, j, DJ, DB, DA, has_DA)
+                       : stream_adjoint<2, 3, 1, 5, false>(h, j, DJ, DB, DA, has_DA);
+    if (pair)
+        return nq == 4 ? stream_adjoint<4, 6, 3, 4, true>(h, j, DJ, DB, DA, has_DA)
+                       : stream_adjoint<4, 6, 3, 5, true>(h, j, DJ, DB, DA, has_DA);
+    return nq == 4 ? stream_adjoint<4, 6, 3, 4, false>(h, j, DJ, DB, DA, has_DA)
+                   : stream_adjoint<4, 6, 3, 5, false>(h, j, DJ, DB, DA, has_DA);
 }
 
 }  // namespace cmd

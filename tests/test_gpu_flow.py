@@ -87,3 +87,43 @@ def test_ssprk53_matches_oracle_at_its_edges(api, oracle, dims, drive):
     np.testing.assert_array_equal(traj[-1][1], api.get_gpu_spins(h))
     for r, (_, s) in enumerate(traj):
         assert np.abs(obs[r, :9] - o.magnetizations(s)).max() <= 1e-13
+
+
+@pytest.mark.parametrize("kind,dims", [("kitaev", (25, 25)), ("kitaev", (38, 64)), ("kitaev", (35, 66)), ("pyro", (5, 5, 5)),
+                                       ("pyro", (6, 6, 6)), ("pyro", (7, 7, 7)), ("pyro", (5, 8, 8)), ("pyro", (8, 8, 8)),
+                                       ("pyro", (4, 4, 4)), ("pyro", (2, 3, 5))])
+def test_cluster_flow_and_paired_bonds_match_oracle(api, oracle, kind, dims):
+    """Lattices over clusters of 2 and 4 CTAs (slabs that cut cell rows, an uneven last slab, the most cells a slab
+    takes) and pyrochlore cells with paired bonds, each with a pulse and a field, three trajectories."""
+    from classical_mcmc_spin_b200.lattice import Lattice
+    if kind == "kitaev":
+        lat, o = Lattice.kitaev(*dims, 1), oracle.OracleLattice.kitaev(*dims, 1)
+    else:
+        kw = dict(h=0.2, Jzz=1.0, Jpm=0.05, Jpmpm=0.02, cubic=True)
+        lat = Lattice.pyrochlore_non_kramer(*dims, field_direction=R111, **kw)
+        o = oracle.OracleLattice.pyrochlore_nk(*dims, direction=R111, **kw)
+    fin = np.tile(R111, lat.N_atoms)
+    fd = lat.rotate_pulse(fin, fin)
+    o.set_pulse(fin, 0.1, fin, 0.3, 0.5, 0.2, 0.7)
+    h = lat.to_gpu()
+    states = np.stack([_spins(lat.lattice_size, 300 + b) for b in range(3)])
+    one = np.ones(3)
+    obs, out = api.run_batch(h, states, 40, 0.01, T0=0.0, save_interval=3, t1=0.1 * one, t2=0.3 * one, a1=0.5 * one,
+                             a2=0.5 * one, d1=fd[:3 * lat.N_atoms], d2=fd[3 * lat.N_atoms:], width=0.2, freq=0.7)
+    for b in range(3):
+        rows, ref = o.md_rk4(states[b], 0.0, 0.395, 0.01, 3, gpu_loop=True)
+        assert len(rows) == obs.shape[1]
+        assert np.abs(obs[b] - rows[:, 1:11]).max() <= 1e-12
+        assert np.abs(out[b] - ref).max() <= 1e-10
+
+
+def test_sliced_cluster_batch_equals_single_runs(api):
+    from classical_mcmc_spin_b200.lattice import Lattice
+    lat = Lattice.kitaev(48, 48, 1)
+    h = lat.to_gpu()
+    states = np.stack([_spins(lat.lattice_size, 500 + b) for b in range(75)])
+    obs, fin = api.run_batch(h, states, 60, 0.01, save_interval=4)
+    for b in (0, 36, 37, 74):
+        o1, f1 = api.run_batch(h, states[b:b + 1], 60, 0.01, save_interval=4)
+        np.testing.assert_array_equal(obs[b], o1[0])
+        np.testing.assert_array_equal(fin[b], f1[0])
