@@ -162,14 +162,17 @@ int cmd_adjoint_rk4(cmd_handle* h, const cmd_adjoint_desc* d) {
         }
     }
     const int64_t B = d->B, S = d->n_steps, N3 = h->N * 3, V = N3;
+    const int cpt = cmd::kStreamTile / std::max(1, h->NA);
+    const int tiles = (int)((h->lay.G + cpt - 1) / cpt);
+    const int64_t Vp = (int64_t)NA * 3 * tiles * cpt;    // a vector of the streamed path, padded to whole tiles
     int64_t C = d->checkpoint_every > 0 ? d->checkpoint_every : (int64_t)std::ceil(std::sqrt((double)S));
     C = std::max<int64_t>(1, std::min(C, S));
     const int64_t K = (S + C - 1) / C;
     const bool fwd_only = d->forward_only != 0;
     if (int rc = h->awork.ensure((size_t)B * 5 * V * sizeof(double))) return rc;
     if (!fwd_only) {
-        if (int rc = h->ackpt.ensure((size_t)B * K * V * sizeof(double))) return rc;
-        if (int rc = h->aseg.ensure((size_t)B * C * 4 * V * sizeof(double))) return rc;
+        if (int rc = h->ackpt.ensure((size_t)B * K * Vp * sizeof(double))) return rc;
+        if (int rc = h->aseg.ensure((size_t)B * C * 4 * Vp * sizeof(double))) return rc;
     }
     if (int rc = h->amloc.ensure((size_t)B * (S + 1) * 3 * sizeof(double))) return rc;
     if (int rc = h->aout.ensure((size_t)B * (1 + kAdjParams) * sizeof(double))) return rc;
@@ -215,8 +218,6 @@ int cmd_adjoint_rk4(cmd_handle* h, const cmd_adjoint_desc* d) {
     a.forward_only = fwd_only;
     // resident (one CTA or cluster per trajectory) when a variant holds the lattice; else one
     // CTA per trajectory in global memory when the batch fills the GPU, else streamed stages
-    const int cpt = cmd::kStreamTile / std::max(1, h->NA);
-    const int tiles = (int)((h->lay.G + cpt - 1) / cpt);
     const int resident = (d->path == CMD_ADJ_AUTO || d->path == CMD_ADJ_RESIDENT) ? pick_adjoint_cluster(h) : -1;
     if (d->path == CMD_ADJ_RESIDENT && resident < 0)
         return fail(CMD_ERR_UNSUPPORTED, "no resident adjoint variant holds this lattice");

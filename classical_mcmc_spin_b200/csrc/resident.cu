@@ -220,6 +220,9 @@ const StageTimes kSSPRK53Times = {
 
 const Variant kVariants[] = {
     // 2-atom cells with 3 bonds per site (Kitaev / Heisenberg honeycomb)
+    // shorter rows for small lattices: more CTAs per SM
+    CMD_FLOW(2, 3, 1, 160, 4, true),
+    CMD_FLOW(2, 3, 1, 288, 2, true),
     CMD_FLOW(2, 3, 1, 640, 1, true),
     CMD_FLOW(2, 3, 1, 640, 1, false),
     CMD_VARIANT(2, 3, 1, 1, 640, 1, true, 1),
@@ -433,7 +436,16 @@ int64_t resident_launches(const ResidentArgs& a, int64_t B) {
 // 2.47 / 1.93 us, 864 cells (two per thread, spills) 8.66 / 2.84 us.
 int batch_variant(const cmd_handle* h, int64_t B, bool drive) {
     const int vi = pick_variant(h);
-    if (vi < 0 || vi == h->variant || kVariants[vi].flow || kVariants[vi].CS > 1) return vi;
+    if (vi < 0 || vi == h->variant || kVariants[vi].CS > 1) return vi;
+    if (kVariants[vi].flow) {
+        // a helper warp can cost a CTA per SM: batches that need the CTA more go without
+        const int64_t slots = kVariants[vi].slots(h, drive);
+        for (int i = vi + 1; i < kNumVariants && kVariants[vi].help && B > slots; ++i) {
+            const Variant& v = kVariants[i];
+            if (v.flow && v.CS == 1 && !v.help && variant_fits(v, h->lay)) return v.slots(h, drive) > slots ? i : vi;
+        }
+        return vi;
+    }
     for (int i = 0; i < kNumVariants; ++i) {
         const Variant& v = kVariants[i];
         if (!v.flow || v.CS == 1 || !variant_fits(v, h->lay)) continue;

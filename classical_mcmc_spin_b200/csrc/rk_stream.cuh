@@ -9,8 +9,11 @@
 // uses the same launches for its segment recompute and one stream_vjp_kernel
 // launch per stage for the reverse sweep (one site per thread).
 //
-// Vectors are cell-major SoA per trajectory, v[(atom*3 + c)*G + g], trajectory
-// b at p + b*stride (SVec).  Per stage a cell reads its stage input (own and
+// Vectors are blocked by tiles of CP = 256 / NAT cells, v[((g / CP)*NAT*3 + atom*3 + c)*CP
+// + g % CP] (soff), the last tile padded, trajectory b at p + b*stride (SVec): a site's
+// components and its in-cell partners lie at compile-time distances, which takes most of
+// the index arithmetic out of the stages (with one row of G cells per component, 140 of a
+// warp's 410 instructions), and a tile is one contiguous piece.  Per stage a cell reads its stage input (own and
 // partners'), y and the RK4 sum, and writes the sum and the next stage input:
 // per spin 72 B (stage 0: y in, sum and next input out), 120 B (stages 1, 2)
 // and 96 B (stage 3: y written in place), 408 B per spin-step when the
@@ -71,6 +74,13 @@ struct StreamArgs {
 template <int NAT>
 constexpr int stream_cells() { return kStreamTile / NAT; }
 
+// Offset of component 0 of site (cell g, atom at) in a vector; component c is c * stream_cells<NAT>() further.
+template <int NAT>
+__host__ __device__ __forceinline__ int soff(int g, int at) {
+    constexpr int CP = stream_cells<NAT>();
+    return g / CP * (NAT * 3 * CP) + at * 3 * CP + g % CP;
+}
+
 template <int NAT>
 __device__ __forceinline__ void stream_site(int& at, int& g) {
     constexpr int CPT = stream_cells<NAT>();
@@ -88,14 +98,15 @@ __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, cons
                                                const double* y, double* acc, double* Ynext, double f1, double f2,
                                                bool drive, double* obs) {
     constexpr int NL = Z - LZ;
-    const long long i0 = (long long)(AT * 3) * G + g;
+    constexpr int CP = stream_cells<NAT>();
+    const int i0 = soff<NAT>(g, AT);
     double S[3], yv[3], av[3], H[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) S[c] = Yin[i0 + c * G];
+    for (int c = 0; c < 3; ++c) S[c] = Yin[i0 + c * CP];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        yv[c] = s == 0 ? S[c] : y[i0 + c * G];
-        av[c] = (s == 0 || !acc) ? 0.0 : acc[i0 + c * G];
+        yv[c] = s == 0 ? S[c] : y[i0 + c * CP];
+        av[c] = (s == 0 || !acc) ? 0.0 : acc[i0 + c * CP];
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) H[d] = cp.has_field ? -cp.field[AT][d] : 0.0;
@@ -107,13 +118,13 @@ __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, cons
     }
 #pragma unroll
     for (int n = 0; n < LZ; ++n) {
-        const long long ip = (long long)(((AT + 1 + n) % NAT) * 3) * G + g;
-        double P0 = Yin[ip], P1 = Yin[ip + G], P2 = Yin[ip + 2 * G];
+        const int ip = i0 + ((AT + 1 + n) % NAT - AT) * 3 * CP;
+        double P0 = Yin[ip], P1 = Yin[ip + CP], P2 = Yin[ip + 2 * CP];
         if constexpr (PAIR) {
             const int p = nbr[(AT * NL + n) * G + g];
             P0 += Yin[p];
-            P1 += Yin[p + G];
-            P2 += Yin[p + 2 * G];
+            P1 += Yin[p + CP];
+            P2 += Yin[p + 2 * CP];
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d)
@@ -124,7 +135,7 @@ __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, cons
         const int n = LZ + m;
         if (n < cp.zc[AT]) {
             const int p = nbr[(AT * NL + m) * G + g];
-            const double P0 = Yin[p], P1 = Yin[p + G], P2 = Yin[p + 2 * G];
+            const double P0 = Yin[p], P1 = Yin[p + CP], P2 = Yin[p + 2 * CP];
 #pragma unroll
             for (int d = 0; d < 3; ++d)
                 bond_acc(H[d], cp.J[AT][n][3 * d], cp.J[AT][n][3 * d + 1], cp.J[AT][n][3 * d + 2], P0, P1, P2);
@@ -132,9 +143,9 @@ __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, cons
     }
     if (OBS == 2) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) obs[3 * AT + c] += S[c];
+        for (int c = 0; c < 3; ++c) obs[c] = S[c];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) obs[3 * NAT] += S[d] * (H[d] - (cp.has_field ? cp.field[AT][d] : 0.0));
+        for (int d = 0; d < 3; ++d) obs[3] += S[d] * (H[d] - (cp.has_field ? cp.field[AT][d] : 0.0));
     }
     if (drive) {
 #pragma unroll
@@ -144,7 +155,7 @@ __device__ __forceinline__ void rk4_stage_site(const Couplings<NAT, Z>& cp, cons
     const double cy = s == 2 ? dt : 0.5 * dt;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const long long i = i0 + c * G;
+        const int i = i0 + c * CP;
         if (s == 0) {
             acc[i] = k[c];
             Ynext[i] = 1.0 * yv[c] + cy * k[c];
@@ -226,27 +237,40 @@ __device__ __forceinline__ bool block_sum_par(double (&v)[NV], double* red, int 
     return true;
 }
 
-// Block-reduces this thread's partial o[NR] and stores it in the tile's slot.
-template <int NR>
-__device__ __forceinline__ void stream_store_partial(const StreamArgs& a, int b, const double (&o)[NR],
-                                                     double* red) {
-    double v[16];
+// Block sums of a site's spin and energy term o[4] (zeros past the last cell), stored in the tile's slot: a warp's
+// sites are one atom, so four values are reduced per warp; value q < 3 NAT adds the warps of its atom, the last one
+// all of them, in warp order.
+template <int NAT>
+__device__ __forceinline__ void stream_store_partial(const StreamArgs& a, int b, double (&o)[4], double* red) {
+    constexpr int NW = kStreamTile / 32, WA = NW / NAT;
+    static_assert(WA >= 1, "an atom fills a warp");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double r = warp_reduce_many<4>(o);
+    if ((lane & 7) == 0) red[warp * 4 + (lane >> 3)] = r;
+    __syncthreads();
+    if (tid > 3 * NAT) return;
+    double t = 0.0;
+    if (tid < 3 * NAT) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = q < NR ? o[q] : 0.0;
-    double t;
-    if (block_sum_par<16>(v, red, NR, &t)) a.part[((long long)b * a.tiles + blockIdx.x) * kPart + threadIdx.x] = t;
+        for (int w = 0; w < WA; ++w) t += red[(tid / 3 * WA + w) * 4 + tid % 3];
+    } else {
+#pragma unroll
+        for (int w = 0; w < NW; ++w) t += red[w * 4 + 3];
+    }
+    a.part[((long long)b * a.tiles + blockIdx.x) * kPart + tid] = t;
 }
 
 // One RK4 stage s of step n for every (tile, trajectory).  Stage 0 also leaves
 // the observables' partials of Yin (= y_n) and the checkpoint of y_n; the
 // first tile of stage 1 finishes step n's observables.
-template <int NAT, int Z, int LZ, bool PAIR>
+// The stage is a template parameter: one kernel for all four carries their code for every
+// atom, and waits for instructions (1.8 of 17 cycles an issue).
+template <int NAT, int Z, int LZ, bool PAIR, int s, bool with_obs>
 __global__ void __launch_bounds__(kStreamTile, 4)
-stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ StreamArgs a, int s,
-                    long long n_arg, SVec Yin, SVec y, SVec acc, SVec Ynext, int with_obs) {
-    constexpr int NR = 3 * NAT + 1;
+stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ StreamArgs a, long long n_arg,
+                    SVec Yin, SVec y, SVec acc, SVec Ynext) {
     const long long n = (a.nbase ? *a.nbase : 0) + n_arg;
-    __shared__ double red[32 * kRedStride];
+    __shared__ double red[kStreamTile / 8];
     __shared__ double tot[16];
     const int b = a.b0 + blockIdx.y;
     int at, g;
@@ -255,9 +279,7 @@ stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_c
     double f1, f2;
     stream_drive(a, b, n, s, f1, f2);
     const bool drive = a.drive != nullptr && (f1 != 0.0 || f2 != 0.0);
-    double o[NR];
-#pragma unroll
-    for (int q = 0; q < NR; ++q) o[q] = 0.0;
+    double o[4] = {0.0, 0.0, 0.0, 0.0};
     if (g < a.G) {
         const double* yin = Yin.at(b);
         with_atom<NAT>(at, [&](auto tag) {
@@ -271,11 +293,11 @@ stream_stage_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_c
             if (s == 0 && a.ckpt && n % a.ckpt_every == 0) {
                 double* dst = a.ckpt + ((long long)b * a.n_ckpt + n / a.ckpt_every) * a.V;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) dst[(long long)(AT * 3 + c) * a.G + g] = yin[(long long)(AT * 3 + c) * a.G + g];
+                for (int c = 0; c < 3; ++c) dst[soff<NAT>(g, AT) + c * stream_cells<NAT>()] = yin[soff<NAT>(g, AT) + c * stream_cells<NAT>()];
             }
         });
     }
-    if (s == 0 && with_obs) stream_store_partial<NR>(a, b, o, red);
+    if (s == 0 && with_obs) stream_store_partial<NAT>(a, b, o, red);
 }
 
 // Advances the step base of a replayed launch sequence by k steps.
@@ -292,14 +314,11 @@ static __global__ void stream_set_base_kernel(long long* nbase, long long v) {
 template <int NAT, int Z, int LZ, bool PAIR>
 __global__ void __launch_bounds__(kStreamTile)
 stream_obs_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ StreamArgs a, SVec y) {
-    constexpr int NR = 3 * NAT + 1;
-    __shared__ double red[32 * kRedStride];
+    __shared__ double red[kStreamTile / 8];
     const int b = a.b0 + blockIdx.y;
     int at, g;
     stream_site<NAT>(at, g);
-    double o[NR];
-#pragma unroll
-    for (int q = 0; q < NR; ++q) o[q] = 0.0;
+    double o[4] = {0.0, 0.0, 0.0, 0.0};
     if (g < a.G) {
         // a stage-3 pass with no output: only the observables of y are kept
         with_atom<NAT>(at, [&](auto tag) {
@@ -307,7 +326,7 @@ stream_obs_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_con
                                                                 nullptr, 0.0, 0.0, false, o);
         });
     }
-    stream_store_partial<NR>(a, b, o, red);
+    stream_store_partial<NAT>(a, b, o, red);
 }
 
 // Finishes step n's observables (one CTA per trajectory).
@@ -329,7 +348,7 @@ __global__ void stream_load_kernel(const double* __restrict__ y0, long long y0_s
 #pragma unroll
     for (int at = 0; at < NAT; ++at)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) dst[(at * 3 + c) * G + g] = src[((long long)g * NAT + at) * 3 + c];
+        for (int c = 0; c < 3; ++c) dst[soff<NAT>(g, at) + c * stream_cells<NAT>()] = src[((long long)g * NAT + at) * 3 + c];
 }
 
 template <int NAT>
@@ -342,7 +361,7 @@ __global__ void stream_store_kernel(SVec y, int G, double* __restrict__ out) {
 #pragma unroll
     for (int at = 0; at < NAT; ++at)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) dst[((long long)g * NAT + at) * 3 + c] = src[(at * 3 + c) * G + g];
+        for (int c = 0; c < 3; ++c) dst[((long long)g * NAT + at) * 3 + c] = src[soff<NAT>(g, at) + c * stream_cells<NAT>()];
 }
 
 // ---------------------------------------------------------------------------
@@ -372,7 +391,8 @@ __global__ void stream_lam_init_kernel(const __grid_constant__ StreamVjpArgs a, 
 #pragma unroll
     for (int at = 0; at < NAT; ++at)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) l[(at * 3 + c) * a.G + g] = 2.0 * (a.mloc[i + c] - a.target[i + c]) / a.n_sites;
+        for (int c = 0; c < 3; ++c)
+            l[soff<NAT>(g, at) + c * stream_cells<NAT>()] = 2.0 * (a.mloc[i + c] - a.target[i + c]) / a.n_sites;
 }
 
 // Hbar of the first VJP stage of a segment: hb = Y x (c lam) of every site.
@@ -383,20 +403,21 @@ stream_hbar_kernel(int G, double c, SVec Y, SVec lam, SVec hb) {
     int at, g;
     stream_site<NAT>(at, g);
     if (g >= G) return;
-    const long long i = (long long)(at * 3) * G + g;
+    constexpr int CP = stream_cells<NAT>();
+    const int i = soff<NAT>(g, at);
     const double *y = Y.at(b) + i, *l = lam.at(b) + i;
     double* o = hb.at(b) + i;
-    const double y0 = y[0], y1 = y[G], y2 = y[2 * G], v0 = c * l[0], v1 = c * l[G], v2 = c * l[2 * G];
+    const double y0 = y[0], y1 = y[CP], y2 = y[2 * CP], v0 = c * l[0], v1 = c * l[CP], v2 = c * l[2 * CP];
     o[0] = y1 * v2 - y2 * v1;
-    o[G] = y2 * v0 - y0 * v2;
-    o[2 * G] = y0 * v1 - y1 * v0;
+    o[CP] = y2 * v0 - y0 * v2;
+    o[2 * CP] = y0 * v1 - y1 * v0;
 }
 
-// Coefficients and outputs of one stage VJP: v = ca lam + cb S of this stage; kind 0 (RK stage 3): S = sbar, acc = lam
+// Coefficients and outputs of one stage VJP: v = ca lam + cb S of this stage (cb 0 for kind 0); kind 0 (RK stage 3): S = sbar, acc = lam
 // + sbar; 1 (stages 2, 1): S = sbar, acc += sbar; 2 (stage 0): lam = acc + sbar + dl.  Then the next VJP stage's
 // Hbar = Ynext x (ca2 lam + cb2 S), unless Ynext is null.
 struct VjpStage {
-    int s, kind;
+    int s;
     double ca, cb, ca2, cb2;
 };
 
@@ -404,7 +425,7 @@ struct VjpStage {
 // stream_hbar_kernel) are read of the partners too, every other vector only at the own site, so lam, S and acc change
 // in place.  Sum over bonds as in vjp_cell; with PAIR (bonds and their parameter derivatives paired) the two partners
 // of a pair are added first.
-template <int NAT, int Z, int LZ, int NQ, int AT, bool PAIR>
+template <int NAT, int Z, int LZ, int NQ, int AT, bool PAIR, int kind>
 __device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, const ParamDerivs<NAT, Z, NQ>& pd,
                                                 const int* __restrict__ nbr, int G, int g, const VjpStage& st,
                                                 const double* __restrict__ Y, const double* __restrict__ hb,
@@ -412,16 +433,17 @@ __device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, con
                                                 double f1, double f2, bool drive, const double (&dl)[3],
                                                 double (&gq)[NQ]) {
     constexpr int NL = Z - LZ;
-    const long long i0 = (long long)(AT * 3) * G + g;
+    constexpr int CP = stream_cells<NAT>();
+    const int i0 = soff<NAT>(g, AT);
     double Yo[3], ho[3], lo[3], so[3], ao[3], yn[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const long long i = i0 + (long long)c * G;
+        const int i = i0 + c * CP;
         Yo[c] = Y[i];
         ho[c] = hb[i];
         lo[c] = lam[i];
-        so[c] = st.kind == 0 ? 0.0 : S[i];
-        ao[c] = st.kind == 0 ? lo[c] : acc[i];
+        so[c] = kind == 0 ? 0.0 : S[i];
+        ao[c] = kind == 0 ? lo[c] : acc[i];
         yn[c] = Ynext ? Ynext[i] : 0.0;
     }
     double H[3], sb[3] = {0.0, 0.0, 0.0};
@@ -463,14 +485,14 @@ __device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, con
     };
 #pragma unroll
     for (int n = 0; n < LZ; ++n) {
-        const long long ip = (long long)(((AT + 1 + n) % NAT) * 3) * G + g;
-        double P[3] = {Y[ip], Y[ip + G], Y[ip + 2 * G]}, Q[3] = {hb[ip], hb[ip + G], hb[ip + 2 * G]};
+        const int ip = i0 + ((AT + 1 + n) % NAT - AT) * 3 * CP;
+        double P[3] = {Y[ip], Y[ip + CP], Y[ip + 2 * CP]}, Q[3] = {hb[ip], hb[ip + CP], hb[ip + 2 * CP]};
         if constexpr (PAIR) {
             const int p = nbr[(AT * NL + n) * G + g];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                P[c] += Y[p + c * G];
-                Q[c] += hb[p + c * G];
+                P[c] += Y[p + c * CP];
+                Q[c] += hb[p + c * CP];
             }
         }
         bond(n, P, Q);
@@ -479,7 +501,7 @@ __device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, con
     for (int m = 0; m < (PAIR ? 0 : NL); ++m)
         if (LZ + m < cp.zc[AT]) {
             const int p = nbr[(AT * NL + m) * G + g];
-            const double P[3] = {Y[p], Y[p + G], Y[p + 2 * G]}, Q[3] = {hb[p], hb[p + G], hb[p + 2 * G]};
+            const double P[3] = {Y[p], Y[p + CP], Y[p + 2 * CP]}, Q[3] = {hb[p], hb[p + CP], hb[p + 2 * CP]};
             bond(LZ + m, P, Q);
         }
     if (drive) {
@@ -490,15 +512,15 @@ __device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, con
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         v[c] = st.ca * lo[c];
-        if (st.cb != 0.0) v[c] = v[c] + st.cb * so[c];
+        if (kind != 0) v[c] = v[c] + st.cb * so[c];
     }
     sb[0] += v[1] * H[2] - v[2] * H[1];
     sb[1] += v[2] * H[0] - v[0] * H[2];
     sb[2] += v[0] * H[1] - v[1] * H[0];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const long long i = i0 + (long long)c * G;
-        if (st.kind == 2) {
+        const int i = i0 + c * CP;
+        if (kind == 2) {
             lo[c] = ao[c] + sb[c] + dl[c];
             lam[i] = lo[c];
         } else {
@@ -506,18 +528,18 @@ __device__ __forceinline__ void stream_vjp_site(const Couplings<NAT, Z>& cp, con
             acc[i] = ao[c] + sb[c];
         }
         v[c] = st.ca2 * lo[c];
-        if (st.cb2 != 0.0) v[c] = v[c] + st.cb2 * sb[c];
+        if (kind != 2) v[c] = v[c] + st.cb2 * sb[c];
     }
     if (Ynext) {
         hb_out[i0] = yn[1] * v[2] - yn[2] * v[1];
-        hb_out[i0 + G] = yn[2] * v[0] - yn[0] * v[2];
-        hb_out[i0 + 2 * G] = yn[0] * v[1] - yn[1] * v[0];
+        hb_out[i0 + CP] = yn[2] * v[0] - yn[0] * v[2];
+        hb_out[i0 + 2 * CP] = yn[0] * v[1] - yn[1] * v[0];
     }
 }
 
 // One stage VJP of step n for every (tile, trajectory), one site per thread (atom uniform per warp, so couplings and
 // derivatives are constant-bank operands); the tile's parameter cotangents are added to its slot.
-template <int NAT, int Z, int LZ, int NQ, bool PAIR>
+template <int NAT, int Z, int LZ, int NQ, bool PAIR, int kind>
 __global__ void __launch_bounds__(kStreamTile, 3)
 stream_vjp_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_constant__ ParamDerivs<NAT, Z, NQ> pd,
                   const __grid_constant__ StreamVjpArgs a, const __grid_constant__ VjpStage st, long long n_arg, SVec Y,
@@ -537,7 +559,7 @@ stream_vjp_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_con
     }
     const bool drive = a.drive != nullptr && (f1 != 0.0 || f2 != 0.0);
     double dl[3] = {0.0, 0.0, 0.0};
-    if (st.kind == 2) {
+    if (kind == 2) {
         const long long i = ((long long)b * (a.n_steps + 1) + n) * 3;
 #pragma unroll
         for (int c = 0; c < 3; ++c) dl[c] = 2.0 * (a.mloc[i + c] - a.target[i + c]) / a.n_sites;
@@ -547,7 +569,7 @@ stream_vjp_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_con
     for (int q = 0; q < NQ; ++q) gq[q] = 0.0;
     if (g < a.G)
         with_atom<NAT>(at, [&](auto tag) {
-            stream_vjp_site<NAT, Z, LZ, NQ, decltype(tag)::value, PAIR>(
+            stream_vjp_site<NAT, Z, LZ, NQ, decltype(tag)::value, PAIR, kind>(
                 cp, pd, a.nbr, a.G, g, st, Y.at(b), hb.at(b), lam.at(b), S.at(b), acc.at(b), Ynext.at(b), hb_out.at(b),
                 f1, f2, drive, dl, gq);
         });
@@ -555,7 +577,9 @@ stream_vjp_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_con
 #pragma unroll
     for (int q = 0; q < NQV; ++q) v[q] = q < NQ ? gq[q] : 0.0;
     double t;
-    if (block_sum_par<NQV>(v, red, NQ, &t)) a.gpart[((long long)b * a.tiles + blockIdx.x) * kPart + threadIdx.x] += t;
+    // one CTA per slot and launch: a reduction without a result is as ordered as a load and a store, and not waited for
+    if (block_sum_par<NQV>(v, red, NQ, &t))
+        atomicAdd(&a.gpart[((long long)b * a.tiles + blockIdx.x) * kPart + threadIdx.x], t);
 }
 
 // grad[b][q] = sum over tiles of the partials, in a fixed order (lane l adds tiles l, l + 32, ..., then a butterfly);

@@ -57,7 +57,9 @@ int run_steps(cmd_handle* h, cudaStream_t st, int64_t S, int64_t groups, const s
     return CMD_OK;
 }
 
-// Partner offsets of the streamed kernels, [NAT][Z-LZ][G] (Layout::nbr, or nbr_pair when `pair`); built on first use.
+// Partner offsets (soff) of the streamed kernels, [NAT][Z-LZ][G], from Layout::nbr or, when `pair`, nbr_pair; built
+// on first use.
+template <int NAT>
 int stream_table(cmd_handle* h, bool pair) {
     DevBuf& d = h->nbrt[pair];
     if (d.p) return CMD_OK;
@@ -68,10 +70,24 @@ int stream_table(cmd_handle* h, bool pair) {
     for (int64_t g = 0; g < L.G; ++g)
         for (int a = 0; a < L.NA; ++a)
             for (int m = 0; m < NL; ++m)
-                t[((size_t)a * NL + m) * L.G + g] = src[((size_t)g * L.NA + a) * NL + m];
+            {
+                const int64_t off = src[((size_t)g * L.NA + a) * NL + m], at = off / (3 * L.G);
+                t[((size_t)a * NL + m) * L.G + g] = soff<NAT>((int)(off - at * 3 * L.G), (int)at);
+            }
     if (int rc = d.ensure(t.size() * sizeof(int))) return rc;
     CUDA_TRY(cudaMemcpy(d.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice));
     return CMD_OK;
+}
+
+// One launch of RK stage s.
+template <int NAT, int Z, int LZ, bool PAIR>
+void stage(int s, dim3 grid, cudaStream_t st, const Couplings<NAT, Z>& cp, const StreamArgs& a, int64_t n, SVec Yin, SVec y,
+           SVec acc, SVec Ynext, int obs) {
+    auto kern = s == 0   ? (obs ? stream_stage_kernel<NAT, Z, LZ, PAIR, 0, true> : stream_stage_kernel<NAT, Z, LZ, PAIR, 0, false>)
+                : s == 1 ? (obs ? stream_stage_kernel<NAT, Z, LZ, PAIR, 1, true> : stream_stage_kernel<NAT, Z, LZ, PAIR, 1, false>)
+                : s == 2 ? stream_stage_kernel<NAT, Z, LZ, PAIR, 2, false>
+                         : stream_stage_kernel<NAT, Z, LZ, PAIR, 3, false>;
+    kern<<<grid, kStreamTile, 0, st>>>(cp, a, n, Yin, y, acc, Ynext);
 }
 
 // Trajectories per group of a streamed run with `vectors` vectors of V doubles each: as many as keep the group's
@@ -103,7 +119,7 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
     int32_t nl = 0;
     const int G = (int)h->lay.G;
     const int tiles = (G + cmd::stream_cells<NAT>() - 1) / cmd::stream_cells<NAT>();
-    const int64_t V = (int64_t)NAT * 3 * G;
+    const int64_t V = (int64_t)NAT * 3 * tiles * cmd::stream_cells<NAT>();      // padded to whole tiles
     const int64_t B = r.B;
     if (B > 65535) return fail(CMD_ERR_UNSUPPORTED, "streamed batches are limited to 65535 trajectories");
     if (r.traj && B != 1) return fail(CMD_ERR_UNSUPPORTED, "streamed state saving is for single trajectories");
@@ -116,7 +132,7 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
     a.G = G;
     a.tiles = tiles;
     a.B = (int)B;
-    if (int rc = stream_table(h, PAIR)) return rc;
+    if (int rc = stream_table<NAT>(h, PAIR)) return rc;
     a.nbr = h->nbrt[PAIR].as<int>();
     a.dt = r.dt;
     a.n_steps = r.n_steps;
@@ -172,10 +188,10 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
     if (r.traj) {                                    // states saved between steps: direct launches
         for (int64_t n = 0; n < r.n_steps; ++n) {
             if (n % r.save == 0) save_traj(n / r.save);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 0, n, y, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 1, n, Ya, y, acc, Yb, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 2, n, Yb, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, a, 3, n, Ya, y, acc, y, with_obs);
+            stage<NAT, Z, LZ, PAIR>(0, grid, st, cp, a, n, y, y, acc, Ya, with_obs);
+            stage<NAT, Z, LZ, PAIR>(1, grid, st, cp, a, n, Ya, y, acc, Yb, with_obs);
+            stage<NAT, Z, LZ, PAIR>(2, grid, st, cp, a, n, Yb, y, acc, Ya, with_obs);
+            stage<NAT, Z, LZ, PAIR>(3, grid, st, cp, a, n, Ya, y, acc, y, with_obs);
             nl += 4;
             if ((n & 1023) == 0) CUDA_TRY(cudaGetLastError());
         }
@@ -200,10 +216,10 @@ int stream_forward(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* la
             cmd::StreamArgs ag = a;
             ag.b0 = (int)(i * per);
             const dim3 gg(tiles, (unsigned)std::min(per, B - i * per));
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 0, k, y, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 1, k, Ya, y, acc, Yb, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 2, k, Yb, y, acc, Ya, with_obs);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 3, k, Ya, y, acc, y, with_obs);
+            stage<NAT, Z, LZ, PAIR>(0, gg, st, cp, ag, k, y, y, acc, Ya, with_obs);
+            stage<NAT, Z, LZ, PAIR>(1, gg, st, cp, ag, k, Ya, y, acc, Yb, with_obs);
+            stage<NAT, Z, LZ, PAIR>(2, gg, st, cp, ag, k, Yb, y, acc, Ya, with_obs);
+            stage<NAT, Z, LZ, PAIR>(3, gg, st, cp, ag, k, Ya, y, acc, y, with_obs);
         };
         if (int rc = run_steps(h, st, r.n_steps, groups, key, enqueue, &nl)) return rc;
         a.nbase = nullptr;                           // the final observation below uses absolute steps
@@ -237,7 +253,7 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
     cudaStream_t st = h->stream;
     const int G = (int)h->lay.G;
     const int tiles = (G + cmd::stream_cells<NAT>() - 1) / cmd::stream_cells<NAT>();
-    const int64_t V = (int64_t)NAT * 3 * G, B = j.B, S = j.S, C = j.C, K = j.K;
+    const int64_t V = (int64_t)NAT * 3 * tiles * cmd::stream_cells<NAT>(), B = j.B, S = j.S, C = j.C, K = j.K;
     if (int rc = h->sbuf.ensure((size_t)5 * B * V * sizeof(double))) return rc;
     if (int rc = h->spart.ensure(((size_t)B * tiles * cmd::kPart + B) * sizeof(double))) return rc;
     if (int rc = h->sgpart.ensure((size_t)B * tiles * cmd::kPart * sizeof(double))) return rc;
@@ -261,7 +277,7 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
     a.G = G;
     a.tiles = tiles;
     a.B = (int)B;
-    if (int rc = stream_table(h, PAIR)) return rc;
+    if (int rc = stream_table<NAT>(h, PAIR)) return rc;
     a.nbr = h->nbrt[PAIR].as<int>();
     a.dt = j.dt;
     a.n_steps = S;
@@ -303,10 +319,10 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
             cmd::StreamArgs ag = af;
             ag.b0 = (int)(i * per);
             const dim3 gg(tiles, (unsigned)std::min(per, B - i * per));
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 0, k, y, y, acc, Ya, 1);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 1, k, Ya, y, acc, Yb, 1);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 2, k, Yb, y, acc, Ya, 1);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<gg, cmd::kStreamTile, 0, st>>>(cp, ag, 3, k, Ya, y, acc, y, 1);
+            stage<NAT, Z, LZ, PAIR>(0, gg, st, cp, ag, k, y, y, acc, Ya, 1);
+            stage<NAT, Z, LZ, PAIR>(1, gg, st, cp, ag, k, Ya, y, acc, Yb, 1);
+            stage<NAT, Z, LZ, PAIR>(2, gg, st, cp, ag, k, Yb, y, acc, Ya, 1);
+            stage<NAT, Z, LZ, PAIR>(3, gg, st, cp, ag, k, Ya, y, acc, y, 1);
         };
         int32_t nl = 0;
         if (int rc = run_steps(h, st, S, groups, key, enqueue, &nl)) return rc;
@@ -358,26 +374,28 @@ int stream_adjoint(cmd_handle* h, const StreamAdjJob& j, const std::vector<doubl
             const int64_t n = nb + jj;
             const cmd::SVec y = slot(jj, 0);
             const cmd::SVec last = jj + 1 < len ? slot(jj + 1, 0) : none;
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 0, n, y, y, acc,
+            stage<NAT, Z, LZ, PAIR>(0, grid, st, cp, sa, n, y, y, acc,
                                                                                    slot(jj, 1), 0);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 1, n, slot(jj, 1), y, acc,
+            stage<NAT, Z, LZ, PAIR>(1, grid, st, cp, sa, n, slot(jj, 1), y, acc,
                                                                                    slot(jj, 2), 0);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 2, n, slot(jj, 2), y, acc,
+            stage<NAT, Z, LZ, PAIR>(2, grid, st, cp, sa, n, slot(jj, 2), y, acc,
                                                                                    slot(jj, 3), 0);
-            cmd::stream_stage_kernel<NAT, Z, LZ, PAIR><<<grid, cmd::kStreamTile, 0, st>>>(cp, sa, 3, n, slot(jj, 3), y, acc,
+            stage<NAT, Z, LZ, PAIR>(3, grid, st, cp, sa, n, slot(jj, 3), y, acc,
                                                                                    last, 0);
         }
         cmd::stream_hbar_kernel<NAT><<<grid, cmd::kStreamTile, 0, st>>>(G, dt / 6.0, slot(len - 1, 3), lam, hb[0]);
         for (int64_t jj = len - 1; jj >= 0; --jj) {
             const int64_t n = nb + jj;
-            auto vjp = cmd::stream_vjp_kernel<NAT, Z, LZ, NQ, PAIR>;
+            auto vjp0 = cmd::stream_vjp_kernel<NAT, Z, LZ, NQ, PAIR, 0>;
+            auto vjp1 = cmd::stream_vjp_kernel<NAT, Z, LZ, NQ, PAIR, 1>;
+            auto vjp2 = cmd::stream_vjp_kernel<NAT, Z, LZ, NQ, PAIR, 2>;
             const double c6 = dt / 6.0, c3 = dt / 3.0;
-            const cmd::VjpStage s3{3, 0, c6, 0.0, c3, dt}, s2{2, 1, c3, dt, c3, 0.5 * dt};
-            const cmd::VjpStage s1{1, 1, c3, 0.5 * dt, c6, 0.5 * dt}, s0{0, 2, c6, 0.5 * dt, c6, 0.0};
-            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s3, n, slot(jj, 3), hb[0], lam, Sv, acc, slot(jj, 2), hb[1]);
-            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s2, n, slot(jj, 2), hb[1], lam, Sv, acc, slot(jj, 1), hb[0]);
-            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s1, n, slot(jj, 1), hb[0], lam, Sv, acc, slot(jj, 0), hb[1]);
-            vjp<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s0, n, slot(jj, 0), hb[1], lam, Sv, acc,
+            const cmd::VjpStage s3{3, c6, 0.0, c3, dt}, s2{2, c3, dt, c3, 0.5 * dt};
+            const cmd::VjpStage s1{1, c3, 0.5 * dt, c6, 0.5 * dt}, s0{0, c6, 0.5 * dt, c6, 0.0};
+            vjp0<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s3, n, slot(jj, 3), hb[0], lam, Sv, acc, slot(jj, 2), hb[1]);
+            vjp1<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s2, n, slot(jj, 2), hb[1], lam, Sv, acc, slot(jj, 1), hb[0]);
+            vjp1<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s1, n, slot(jj, 1), hb[0], lam, Sv, acc, slot(jj, 0), hb[1]);
+            vjp2<<<grid, cmd::kStreamTile, 0, st>>>(cp, pd, sv, s0, n, slot(jj, 0), hb[1], lam, Sv, acc,
                                                   jj > 0 ? slot(jj - 1, 3) : none, hb[0]);
         }
     };
