@@ -447,7 +447,7 @@ int cmd_destroy(cmd_handle* h) {
                       &h->pulses, &h->scratch, &h->dframes, &h->dafm, &h->times, &h->drive, &h->raw,
                       &h->tune_states, &h->tune_obs, &h->gwork, &h->gmeta, &h->gstat, &h->grows, &h->gqueue,
                       &h->awork, &h->ackpt, &h->aseg, &h->amloc, &h->aout, &h->ameta, &h->ain,
-                      &h->sbuf, &h->spart, &h->sgpart, &h->snbase, &h->mid, &h->nbrp, &h->nbrt[0], &h->nbrt[1], &h->fctab[2], &h->fctab[4], &h->chunk_states, &h->chunk_rows, &h->cnbr2, &h->cnbr4, &h->cnbr8, &h->cnbr16, &h->cnbr_all, &h->cpush})
+                      &h->sbuf, &h->spart, &h->sgpart, &h->snbase, &h->nbrp, &h->nbrt[0], &h->nbrt[1], &h->fctab[2], &h->fctab[4], &h->chunk_states, &h->chunk_rows, &h->cnbr2, &h->cnbr4, &h->cnbr8, &h->cnbr16, &h->cnbr_all, &h->cpush})
         b->release();
     h->hstage.release();
     h->hfault.release();

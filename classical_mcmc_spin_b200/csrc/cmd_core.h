@@ -86,7 +86,6 @@ struct cmd_handle {
     cmd::DevBuf nbrp;           // Layout::nbr_pair
     cmd::DevBuf fctab[5];       // Layout::flow_cluster: pw, push, peers in one buffer, by cluster size
     cmd::DevBuf nbrt[2];        // partner offsets of the streamed kernels (rk_stream.cuh), unpaired and paired
-    cmd::DevBuf mid;            // states between the slices of a resident batch
     cmd::DevBuf chunk_states, chunk_rows;   // cmd_run_batch: ping-pong states and row buffers of time chunks
     cmd::DevBuf cnbr2, cnbr4, cnbr8, cnbr16;  // partner tables of the 2-, 4-, 8- and 16-CTA cluster kernels
     cmd::DevBuf cnbr_all;       // RK45 on-chip kernels: every slot's partner word per site (built on first use)

@@ -303,6 +303,10 @@ bool plan_tiles(cmd_mixed* h, int cs, const KindTables& k2, const KindTables& k3
             for (int s = lo; s < hi; ++s) {
                 std::vector<Slot> sl, three;
                 slots_of(kind, s, sl, three);
+                // by coupling, so that sites whose tables list the same bonds in another order share tiles
+                auto by_frag = [](const Slot& x, const Slot& y) { return x.frag < y.frag; };
+                std::stable_sort(sl.begin(), sl.end(), by_frag);
+                std::stable_sort(three.begin(), three.end(), by_frag);
                 const int n8 = (int)sl.size();
                 sl.insert(sl.end(), three.begin(), three.end());
                 std::vector<int> key{s % NA, kind == 3 ? f3 + 8 * k3.fi[s] : f2 + 3 * k2.fi[s], n8};

@@ -505,15 +505,12 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
         a.drive = h->drive.as<double>();
     }
     if (r.obs && V.NAT != 2 && V.NAT != 4) return fail(CMD_ERR_UNSUPPORTED, "no row finisher for this cell size");
-    plan_slices(h, V, r.B, r.n_steps, a);
-    // one shared initial state that the results overwrite is read by every trajectory's start
-    if (r.y0_stride == 0 && r.y_out && r.y0 >= r.y_out && r.y0 < r.y_out + r.B * h->N * 3) a.slices = 1;
-    if (a.slices > 1) {
-        if (!r.y_out) {
-            if (int rc = h->mid.ensure((size_t)r.B * h->N * 3 * sizeof(double))) return rc;
-        }
-        a.y_mid = r.y_out ? r.y_out : h->mid.as<double>();
-    }
+    // slices keep their states in the caller's final states (nothing of the handle's: calls without a drive may
+    // overlap on several streams); one shared initial state that those overwrite is read by every trajectory's start
+    const bool over = r.y0_stride == 0 && r.y_out && r.y0 >= r.y_out && r.y0 < r.y_out + r.B * h->N * 3;
+    a.slices = 1;
+    if (r.y_out && !over) plan_slices(h, V, r.B, r.n_steps, a);
+    a.y_mid = r.y_out;
     static const std::vector<double> zeros(3 * 64, 0.0);
     const double* d1 = r.d1 ? r.d1 : zeros.data();
     const double* d2 = r.d2 ? r.d2 : zeros.data();

@@ -29,8 +29,8 @@
 // the issue port 910 of the stage's 1330 cycles there (0.68 us; 0.88 us with a CTA barrier per stage and 205
 // instructions).  B200, 1965 MHz: 768 driven trajectories x 2000 steps 32.1 ms (45.5 ms with the barrier and whole
 // waves; 36.9 ms with whole waves); one trajectory 2.80 us per step (3.61); 40 trajectories of 8x8 x 500 steps
-// 0.95 ms (1.35); 200 of the 1024-spin pyrochlore x 800 driven steps 5.27 ms (11.6; atoms interleaved 1.03 us per
-// stage against 1.71); one 24x24 SSPRK53 trajectory x 400 steps, 11 states saved, 1.59 ms (7.05 in global memory,
+// 0.95 ms (1.35); 200 of the 1024-spin pyrochlore x 800 driven steps 4.35 ms (11.6 with the atoms in sequence; 5.27
+// without paired bonds); one 24x24 SSPRK53 trajectory x 400 steps, 11 states saved, 1.59 ms (7.05 in global memory,
 // where every RK vector is read and written each stage).  Polling progress words instead of waiting on mbarriers: 256 instructions, 0.83 us.
 #pragma once
 

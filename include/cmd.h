@@ -36,7 +36,7 @@ enum {
     CMD_ERR_UNSUPPORTED = 2,
     CMD_ERR_CUDA = 3,
     CMD_ERR_NONFINITE = 4,
-    CMD_ERR_WATCHDOG = 5,
+    CMD_ERR_WATCHDOG = 5,      /* a bounded wait inside a kernel gave up: results invalid */
     CMD_ERR_OOM = 6,
     CMD_ERR_STATE = 7
 };
@@ -245,8 +245,8 @@ int cmd_nonlinear_spectrum(const double* M0, const double* M1, const double* M01
 /* Lattice layout chosen at cmd_create (for diagnostics and the autotuner):
  * info[0] = sites per group (unit-cell atoms), info[1] = groups,
  * info[2] = max bonds per site kept, info[3] = threads per block of the
- * resident RK4 kernel, info[4] = groups per thread, info[5] = shared-memory
- * bytes per trajectory. */
+ * resident RK4 kernel that hold groups, info[4] = groups per thread, info[5] =
+ * shared-memory bytes per trajectory (cluster kernels: of a CTA's own groups). */
 int cmd_layout_info(cmd_handle* h, int64_t* info);
 
 /*
@@ -340,9 +340,9 @@ int cmd_autotune(cmd_handle* h, int64_t B, int64_t n_steps, int32_t* best, doubl
 
 /*
  * CUDA graphs, on by default.  Streamed RK4 (lattices no resident kernel
- * holds; one launch per RK stage): the stage launches of a chunk of 128 steps
- * are captured once as a CUDA graph, kept in the handle and replayed, so a
- * 2x10^4-step run makes 157 graph launches instead of 8x10^4 kernel launches.
+ * holds; one launch per RK stage and group of trajectories): the stage launches
+ * of a chunk of steps (128 divided by the number of groups) are captured once as
+ * a CUDA graph, kept in the handle and replayed.
  * Batched resident runs (drive table, resident kernel, row finisher) and
  * uneven batches (the per-lattice launches on the handle's auxiliary streams,
  * forked from and joined to the call's stream): each call is captured and

@@ -127,3 +127,30 @@ def test_sliced_cluster_batch_equals_single_runs(api):
         o1, f1 = api.run_batch(h, states[b:b + 1], 60, 0.01, save_interval=4)
         np.testing.assert_array_equal(obs[b], o1[0])
         np.testing.assert_array_equal(fin[b], f1[0])
+
+
+@pytest.mark.parametrize("dims", [(2, 3, 4), (6, 5, 9), (13, 13, 13)])
+def test_unpaired_pyrochlore_bonds(api, dims):
+    """Breathing pyrochlore (bonds that leave the cell weaker, so nothing is paired): one CTA, a cluster, streamed;
+    against RK4 over the flat tables in numpy, states to 1e-12 over 12 steps."""
+    from classical_mcmc_spin_b200.lattice import Lattice
+    lat = Lattice.pyrochlore_non_kramer(*dims, h=0.2, field_direction=R111, Jzz=1.0, Jpm=0.05, Jpmpm=0.02)
+    N, z, e = lat.lattice_size, lat.num_bi, lat.export()
+    part = e["partners"].reshape(N, z)
+    J = e["bilinear"].reshape(N, z, 3, 3) * np.where(part // 4 == np.arange(N)[:, None] // 4, 1.0, 0.7)[..., None, None]
+    assert (e["counts"] == z).all()
+    h = api.create_gpu_lattice_data(N, 3, 4, z, e["field"], e["onsite"], J, part, e["counts"], e["frames"], e["afm"])
+    B = e["field"].reshape(N, 3)
+    f = lambda y: np.cross(np.einsum("nzij,nzj->ni", J, y[part]) - B, y)
+    s0 = _spins(N, 77)
+    y, dt = s0.reshape(N, 3).copy(), 0.02
+    for _ in range(12):
+        k1 = f(y)
+        k2 = f(y + 0.5 * dt * k1)
+        k3 = f(y + 0.5 * dt * k2)
+        k4 = f(y + dt * k3)
+        y = y + (dt / 6.0) * (k1 + 2.0 * k2 + 2.0 * k3 + k4)
+    api.set_gpu_spins(h, s0)
+    _, obs, _ = api.integrate_gpu(h, 0.0, 11.5 * dt, dt, 5, "rk4", with_states=False)
+    assert np.abs(api.get_gpu_spins(h) - y.ravel()).max() <= 1e-12
+    assert np.abs(obs[-1, 3:6] - y.mean(0)).max() <= 1e-13
