@@ -648,7 +648,8 @@ int cmd_integrate(cmd_handle* h, double T0, double T1, double dt, int64_t save_i
     const int64_t rows = rows_for(n, save_interval);
     if (rows_out) *rows_out = rows;
     if (max_rows < rows) return fail(CMD_ERR_INVALID_ARG, "max_rows too small");
-    if ((method == CMD_RK4 && rk4_fits(h)) || resident_method(h, method)) {
+    // SSPRK53's envelope table grows with the steps: where it finds no room, the kernel in global memory needs none
+    if ((method == CMD_RK4 && rk4_fits(h)) || (resident_method(h, method) && stages_room(h, n))) {
         if (int rc = run_single(h, T0, dt, n, save_interval, (double)h->N, obs != nullptr, states != nullptr, true,
                                 method))
             return rc;

@@ -258,6 +258,7 @@ int default_variant(const Layout& L);
 int prepare_variant(cmd_handle* h, int vi);
 int pick_variant(const cmd_handle* h);
 int flow_variant(const Layout& L);
+bool stages_room(cmd_handle* h, int64_t n_steps);
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches);
 // Sets a.slices / a.slots of a resident batch (a.drive set); the caller provides a.y_mid when a.slices > 1.
 void plan_slices(const cmd_handle* h, const Variant& V, int64_t B, int64_t n_steps, ResidentArgs& a);

@@ -454,6 +454,17 @@ int batch_variant(const cmd_handle* h, int64_t B, bool drive) {
     return vi;
 }
 
+// Room for the envelope table of n_steps driven SSPRK53 steps.
+bool stages_room(cmd_handle* h, int64_t n_steps) {
+    if (h->amp == 0.0 || n_steps <= 0) return true;
+    if (h->times.ensure((size_t)n_steps * sizeof(double)) == CMD_OK &&
+        h->drive.ensure((size_t)n_steps * 2 * kSSPRK53Times.n * sizeof(double)) == CMD_OK)
+        return true;
+    cudaGetLastError();
+    clear_error();
+    return false;
+}
+
 // Launches drive-table pre-pass (when driven), the resident kernel and the
 // row-finishing post-pass on `st`.  Asynchronous; returns the launch count.
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches) {
