@@ -34,6 +34,7 @@
 // where every RK vector is read and written each stage).  Polling progress words instead of waiting on mbarriers: 256 instructions, 0.83 us.
 #pragma once
 
+#include "flow_wait.h"
 #include "rk4_resident.cuh"
 
 namespace cmd {
@@ -115,12 +116,13 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     double* red = smem + 2 * SB;                     // [kFlowRows][NW][NV] observable partials of the warps
     double* bars = red + flow_ring_doubles(NAT, MAXT);              // [2][NW] inputs, [kFlowRows] full, free
     int* dep = reinterpret_cast<int*>(bars + 2 * NW + 2 * kFlowRows);  // [32] warps a warp exchanges spins with
+    FlowWait* fw = reinterpret_cast<FlowWait*>(dep + 32);
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int ncw = HELP ? nwarps - 1 : nwarps;      // warps with cells
     const uint32_t bar_in = (uint32_t)__cvta_generic_to_shared(bars);
     const uint32_t bar_full = bar_in + 16 * NW, bar_free = bar_full + 8 * kFlowRows;
-    const uint32_t dead = (uint32_t)__cvta_generic_to_shared(dep + 32);
+    const uint32_t dead = (uint32_t)__cvta_generic_to_shared(&fw->dead);
 
     // this CTA's trajectory and steps [n0, n1): items are (slice, trajectory), trajectories fastest
     const long long item = a.item0 + blockIdx.x;
@@ -134,7 +136,8 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     double y[NAT][3], acc[NAT][3], yc[NAT][3];
     int pb[NAT][NL > 0 ? NL : 1];                    // word offset of each partner's component 0 in buffer 0
     const double* y0 = slice == 0 ? a.y0 + b * a.y0_stride : a.y_mid + b * N3;
-    if (tid < 33) dep[tid] = 0;
+    if (tid < 32) dep[tid] = 0;
+    flow_wait_init(fw, tid);
 #pragma unroll
     for (int at = 0; at < NAT; ++at)
 #pragma unroll

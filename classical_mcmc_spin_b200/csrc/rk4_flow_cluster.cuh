@@ -110,7 +110,8 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
     const uint32_t bar_in = (uint32_t)__cvta_generic_to_shared(bars);
     const uint32_t bar_full = bar_in + 16 * NW, bar_free = bar_full + 8 * kFlowRows;
     const uint32_t bar_tot = bar_free + 8 * kFlowRows, bar_tfree = bar_tot + 8 * kFlowRows;
-    const uint32_t dead = bar_tfree + 8 * kFlowRows;
+    FlowWait* fw = reinterpret_cast<FlowWait*>(bars + 2 * NW + 4 * kFlowRows);
+    const uint32_t dead = (uint32_t)__cvta_generic_to_shared(&fw->dead);
 
     // this CTA's trajectory and steps [n0, n1): items are (slice, trajectory), trajectories fastest
     const long long item = a.item0 + blockIdx.x / CS;
@@ -165,7 +166,7 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
         mbar_init(bar_tot + 8 * tid, CS);
         mbar_init(bar_tfree + 8 * tid, 1);
     }
-    if (tid == 0) asm volatile("st.shared.u32 [%0], 0;" ::"r"(dead) : "memory");
+    flow_wait_init(fw, tid);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     flow_cluster_sync();                             // every CTA's barriers exist
     const uint32_t my_in = bar_in + 8 * warp;
