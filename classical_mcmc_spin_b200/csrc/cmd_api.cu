@@ -1234,6 +1234,14 @@ int cmd_set_graphs(cmd_handle* h, int32_t enable) {
     return CMD_OK;
 }
 
+int cmd_set_wait_limit(cmd_handle* h, int64_t ns) {
+    cmd::clear_error();
+    if (int rc = check_handle(h, false)) return rc;
+    if (ns < 0) return fail(CMD_ERR_INVALID_ARG, "negative wait limit");
+    h->wait_ns = ns;
+    return CMD_OK;
+}
+
 int cmd_rk45_variant_count(void) { return rk45_variant_count(); }
 
 int cmd_rk45_variant_info(cmd_handle* h, int32_t idx, char* name, int32_t name_len, int32_t* fits) {

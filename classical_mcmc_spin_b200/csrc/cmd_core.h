@@ -25,6 +25,7 @@
 
 #include "cmd.h"
 #include "cmd_internal.h"
+#include "flow_wait.h"
 #include "rk4_resident.cuh"
 #include "rk_global.cuh"
 
@@ -93,6 +94,7 @@ struct cmd_handle {
     int cnbr_all_cs = 0;        // 2 * cluster size (+1 for halo words) cnbr_all / cpush were built for
     cudaStream_t copy_stream = nullptr;  // cmd_run_batch: device-to-host copies of finished chunks
     cmd::HostBuf hfault;        // one int, page-locked: set by a kernel whose bounded wait gave up
+    int64_t wait_ns = cmd::kWaitLimitNs;   // limit of those waits (cmd_set_wait_limit)
     cmd::HostBuf hstage;        // cmd_run_uneven: page-locked staging of the rows and final states
     std::vector<cudaStream_t> aux_streams;   // concurrent launches of an uneven batch (created on first use)
     // streamed RK4: the stage launches of one chunk of steps captured as a CUDA

@@ -81,6 +81,7 @@ int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double
     cmd::ResidentArgs a = args;
     a.B = B;
     a.fault = h->hfault.as<int>();
+    a.wait_ns = (unsigned long long)h->wait_ns;
     if (h->lay.paired) a.nbr = h->nbrp.as<int>();
     // items are (slice, trajectory), trajectories fastest: the earlier slice of an item ran in an earlier launch
     // (slots <= B), so stream order is the only dependence
@@ -147,6 +148,7 @@ int launch_flow_cluster(const cmd_handle* h, const cmd::ResidentArgs& args, cons
     cmd::ResidentArgs a = args;
     a.B = B;
     a.fault = h->hfault.as<int>();
+    a.wait_ns = (unsigned long long)h->wait_ns;
     FlowClusterArgs fc{};
     const Layout::FlowCluster& t = h->lay.flow_cluster[CS];
     fc.Gc = (int)cluster_cells(h->lay.G, CS);

@@ -22,7 +22,7 @@
 //   * The field sums of a cell's atoms are interleaved (3 NAT independent chains); -B and
 //     2 A S are formed from values the compiler cannot hoist, which keeps every coupling a
 //     constant-bank operand without a branch per atom.
-// Waits are bounded (mbar_wait).
+// Waits are bounded (mbar_wait); a run whose wait gave up skips its remaining steps and reports CMD_ERR_WATCHDOG.
 //
 // Bound: issue slots and the FP64 pipe.  24x24 honeycomb, one step's observables every step: 182 warp instructions
 // per warp and stage, 82 of them FP64; 18 warps put 5 on two of the SM's four schedulers, so the pipe needs 820 and
@@ -69,31 +69,50 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar, bool on) {
         "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t"
         "@p mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"((unsigned)on) : "memory");
 }
-// Waits until the phase of `parity` of the mbarrier completes (acquire).  Bounded: a thread that has waited for
-// 2^30 ns, or sees that another of the CTA gave up (*dead, shared), records it there and in *fault (host) and ends.
-// One block of inline PTX: as a call, or as C++ after a failed first try, the cold path costs the hot one spills.
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t dead, int* fault) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .u64 t0, t1;\n\t.reg .u32 d;\n\t"
-        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%0], %1;\n\t"
-        "@p bra DONE;\n\t"
-        "mov.u64 t0, %globaltimer;\n"
-        "AGAIN:\n\t"
-        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%0], %1, 2000;\n\t"
-        "@p bra DONE;\n\t"
-        "mov.u64 t1, %globaltimer;\n\t"
-        "sub.u64 t1, t1, t0;\n\t"
-        "ld.volatile.shared::cta.u32 d, [%2];\n\t"
-        "setp.gt.u64 p, t1, 1073741824;\n\t"
-        "@p bra GIVEUP;\n\t"
-        "setp.eq.u32 p, d, 0;\n\t"
-        "@p bra AGAIN;\n"
-        "GIVEUP:\n\t"
-        "mov.u32 d, 1;\n\t"
-        "st.volatile.shared::cta.u32 [%2], d;\n\t"
-        "st.volatile.global.u32 [%3], d;\n\t"
-        "exit;\n"
-        "DONE:\n\t}" ::"r"(bar), "r"(parity), "r"(dead), "l"(fault) : "memory");
+// Waits until the phase of `parity` of the mbarrier completes (acquire, at the named scope).  Bounded: a thread that
+// has tried kWaitTries times and for longer than FlowWait::ns (the tries too, so that time in which the GPU runs another
+// process does not count) sets FlowWait::dead and *fault (host) and goes on, as does one that finds `dead` set; every
+// warp of the CTA looks at `dead` once a step and leaves the step loop (gave_up).  No thread ends early: a CTA of a
+// cluster stays while others may store into it, and every thread meets the barriers after the loop.  One block of
+// inline PTX: as a call, or as C++ after a failed first try, the cold path costs the hot one spills.
+constexpr unsigned kWaitTries = 4096;
+#define CMD_MBAR_WAIT(SCOPE)                                                                                 \
+    asm volatile(                                                                                            \
+        "{\n\t.reg .pred p;\n\t.reg .u64 t0, t1, lim;\n\t.reg .u32 d, n;\n\t"                               \
+        "mbarrier.try_wait.parity.acquire." SCOPE ".shared::cta.b64 p, [%0], %1;\n\t"                        \
+        "@p bra DONE;\n\t"                                                                                   \
+        "mov.u64 t0, %%globaltimer;\n\t"                                                                     \
+        "mov.u32 n, 0;\n"                                                                                    \
+        "AGAIN:\n\t"                                                                                         \
+        "ld.volatile.shared::cta.u32 d, [%2];\n\t"                                                           \
+        "setp.ne.u32 p, d, 0;\n\t"                                                                           \
+        "@p bra DONE;\n\t"                                                                                   \
+        "mbarrier.try_wait.parity.acquire." SCOPE ".shared::cta.b64 p, [%0], %1, 2000;\n\t"                  \
+        "@p bra DONE;\n\t"                                                                                   \
+        "add.u32 n, n, 1;\n\t"                                                                               \
+        "mov.u64 t1, %%globaltimer;\n\t"                                                                     \
+        "sub.u64 t1, t1, t0;\n\t"                                                                            \
+        "ld.shared::cta.u64 lim, [%2+8];\n\t"                                                                \
+        "setp.le.u64 p, t1, lim;\n\t"                                                                        \
+        "@p bra AGAIN;\n\t"                                                                                  \
+        "setp.lt.u32 p, n, %4;\n\t"                                                                          \
+        "@p bra AGAIN;\n\t"                                                                                  \
+        "mov.u32 d, 1;\n\t"                                                                                  \
+        "st.volatile.shared::cta.u32 [%2], d;\n\t"                                                           \
+        "st.volatile.global.u32 [%3], d;\n"                                                                  \
+        "DONE:\n\t}"                                                                                         \
+        :                                                                                                    \
+        : "r"(bar), "r"(parity), "r"(words), "l"(fault), "n"(kWaitTries)                                     \
+        : "memory")
+
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t words, int* fault) {
+    CMD_MBAR_WAIT("cta");
+}
+// Whether a wait of the CTA gave up, the same answer in every lane of the warp.
+__device__ __forceinline__ bool gave_up(uint32_t words) {
+    unsigned d;
+    asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(d) : "r"(words));
+    return __any_sync(0xffffffffu, d != 0);
 }
 
 // Stages per step: classic RK4, or the reference GPU's default method SSPRK(5,3) (integrator.cuh:406-448).
@@ -111,7 +130,8 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     constexpr int GS = MAXT;                         // component stride in shared memory
     constexpr int SB = NAT * 3 * GS;                 // one stage buffer
     constexpr int span = 32 / NV;
-    static_assert(flow_ring_doubles(NAT, MAXT) + 2 * NW + 2 * kFlowRows + 17 <= 32 * kRedStride + 12, "ring and barriers fit");
+    static_assert(flow_ring_doubles(NAT, MAXT) + 2 * NW + 2 * kFlowRows + 16 + sizeof(FlowWait) / 8 <= 32 * kRedStride + 12,
+                  "ring, barriers, peer masks and wait words fit");
     extern __shared__ double smem[];
     double* red = smem + 2 * SB;                     // [kFlowRows][NW][NV] observable partials of the warps
     double* bars = red + flow_ring_doubles(NAT, MAXT);              // [2][NW] inputs, [kFlowRows] full, free
@@ -122,7 +142,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     const int ncw = HELP ? nwarps - 1 : nwarps;      // warps with cells
     const uint32_t bar_in = (uint32_t)__cvta_generic_to_shared(bars);
     const uint32_t bar_full = bar_in + 16 * NW, bar_free = bar_full + 8 * kFlowRows;
-    const uint32_t dead = (uint32_t)__cvta_generic_to_shared(&fw->dead);
+    const uint32_t wait_words = (uint32_t)__cvta_generic_to_shared(fw);
 
     // this CTA's trajectory and steps [n0, n1): items are (slice, trajectory), trajectories fastest
     const long long item = a.item0 + blockIdx.x;
@@ -137,7 +157,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     int pb[NAT][NL > 0 ? NL : 1];                    // word offset of each partner's component 0 in buffer 0
     const double* y0 = slice == 0 ? a.y0 + b * a.y0_stride : a.y_mid + b * N3;
     if (tid < 32) dep[tid] = 0;
-    flow_wait_init(fw, tid);
+    flow_wait_init(fw, tid, a.wait_ns);
 #pragma unroll
     for (int at = 0; at < NAT; ++at)
 #pragma unroll
@@ -181,7 +201,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     const bool peer = lane < ncw && warp < ncw && (((dep[warp] | (1 << warp)) >> lane) & 1);
     const uint32_t my_in = bar_in + 8 * warp, peer_in = bar_in + 8 * lane;
     // Stage k (counted over the run) waits for phase k / 2 of input barrier k % 2.
-    auto wait_in = [&](int k) { mbar_wait(my_in + 8 * NW * (k & 1), (k >> 1) & 1, dead, a.fault); };
+    auto wait_in = [&](int k) { mbar_wait(my_in + 8 * NW * (k & 1), (k >> 1) & 1, wait_words, a.fault); };
     auto publish = [&](int k) {                      // the input of stage k is stored
         __syncwarp();
         mbar_arrive(peer_in + 8 * NW * (k & 1), peer);
@@ -278,7 +298,8 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     double part[NV];
     if (HELP && warp == ncw) {
         for (long long n = n0 + save_left; n < n1; n += a.save_every, ++row) {
-            mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, dead, a.fault);
+            mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
+            if (gave_up(wait_words)) break;
             finish_row(row % kFlowRows, row0 + row);
         }
     } else {
@@ -288,6 +309,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
             save_left = observe ? a.save_every - 1 : save_left - 1;
             const bool driven = DRIVE && __any_sync(0xffffffffu, cur_f != 0.0);   // 0*d adds exactly 0
             double next_f = 0.0;
+            bool leave = false;
             if (stager && step + 1 < n1) next_f = dtab[(step + 1) * NE];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
@@ -295,7 +317,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
                 const int rb = k & 1;                // buffer read in this stage; the other one is written
                 const int ti = NS == kFlowSSPRK53 ? s : (s == 0 ? 0 : (s == 3 ? 2 : 1));
                 if (s == 1 && observe) {
-                    mbar_wait(bar_free + 8 * (row % kFlowRows), ((row / kFlowRows) & 1) ^ 1, dead, a.fault);
+                    mbar_wait(bar_free + 8 * (row % kFlowRows), ((row / kFlowRows) & 1) ^ 1, wait_words, a.fault);
                     store_partials(part, row % kFlowRows);
                 }
                 const double(&S)[NAT][3] = s == 0 ? y : yc;
@@ -352,19 +374,21 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
                         wbuf[(at * 3 + c) * GS + g] = s == NS - 1 ? y[at][c] : yc[at][c];
                     }
                 publish(k + 1);
+                if (s == NS - 2) leave = gave_up(wait_words);      // here, where the next wait hides it
             }
             cur_f = next_f;
             if (NS % 4 != 0) k0 = (k0 + NS) & 3;
             if (observe) {
                 if (!HELP) {
                     if (warp == finisher) {
-                        mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, dead, a.fault);
+                        mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
                         finish_row(row % kFlowRows, row0 + row);
                     }
                     finisher = finisher + 1 == ncw ? 0 : finisher + 1;
                 }
                 ++row;
             }
+            if (leave) break;
         }
     }
     __syncthreads();

@@ -36,7 +36,7 @@ struct FlowClusterArgs {
 __host__ __device__ constexpr int flow_halo(int nat) { return nat <= 2 ? 128 : 256; }
 __host__ __device__ constexpr long long flow_cluster_smem_doubles(int nat, int maxt, int cs) {
     return 2LL * nat * 3 * (maxt + flow_halo(nat)) + flow_ring_doubles(nat, maxt) + kFlowRows * cs * flow_nv(nat) +
-           2LL * (maxt / 32) + 4 * kFlowRows + 2;
+           2LL * (maxt / 32) + 4 * kFlowRows + (long long)sizeof(FlowWait) / 8;
 }
 
 __device__ __forceinline__ uint32_t flow_map(uint32_t local, int rank) {
@@ -58,31 +58,9 @@ __device__ __forceinline__ void flow_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// mbar_wait with cluster-scope acquire.  Bounded: a thread that has waited for
-// 2^30 ns, or sees that another of the CTA gave up (*dead, shared), records it there and in *fault (host) and ends.
-// One block of inline PTX: as a call, or as C++ after a failed first try, the cold path costs the hot one spills.
-__device__ __forceinline__ void mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t dead, int* fault) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .u64 t0, t1;\n\t.reg .u32 d;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t"
-        "@p bra DONE;\n\t"
-        "mov.u64 t0, %globaltimer;\n"
-        "AGAIN:\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1, 2000;\n\t"
-        "@p bra DONE;\n\t"
-        "mov.u64 t1, %globaltimer;\n\t"
-        "sub.u64 t1, t1, t0;\n\t"
-        "ld.volatile.shared::cta.u32 d, [%2];\n\t"
-        "setp.gt.u64 p, t1, 1073741824;\n\t"
-        "@p bra GIVEUP;\n\t"
-        "setp.eq.u32 p, d, 0;\n\t"
-        "@p bra AGAIN;\n"
-        "GIVEUP:\n\t"
-        "mov.u32 d, 1;\n\t"
-        "st.volatile.shared::cta.u32 [%2], d;\n\t"
-        "st.volatile.global.u32 [%3], d;\n\t"
-        "exit;\n"
-        "DONE:\n\t}" ::"r"(bar), "r"(parity), "r"(dead), "l"(fault) : "memory");
+// mbar_wait with cluster-scope acquire.
+__device__ __forceinline__ void mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t words, int* fault) {
+    CMD_MBAR_WAIT("cluster");
 }
 
 template <int NAT, int Z, int LZ, int CS, int MAXT, bool STAT, bool DRIVE, bool PAIR>
@@ -111,7 +89,7 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
     const uint32_t bar_full = bar_in + 16 * NW, bar_free = bar_full + 8 * kFlowRows;
     const uint32_t bar_tot = bar_free + 8 * kFlowRows, bar_tfree = bar_tot + 8 * kFlowRows;
     FlowWait* fw = reinterpret_cast<FlowWait*>(bars + 2 * NW + 4 * kFlowRows);
-    const uint32_t dead = (uint32_t)__cvta_generic_to_shared(&fw->dead);
+    const uint32_t wait_words = (uint32_t)__cvta_generic_to_shared(fw);
 
     // this CTA's trajectory and steps [n0, n1): items are (slice, trajectory), trajectories fastest
     const long long item = a.item0 + blockIdx.x / CS;
@@ -166,7 +144,7 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
         mbar_init(bar_tot + 8 * tid, CS);
         mbar_init(bar_tfree + 8 * tid, 1);
     }
-    flow_wait_init(fw, tid);
+    flow_wait_init(fw, tid, a.wait_ns);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     flow_cluster_sync();                             // every CTA's barriers exist
     const uint32_t my_in = bar_in + 8 * warp;
@@ -193,8 +171,8 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
     push_all(0, y);
     // Stage k (counted over the run) waits for phase k / 2 of input barrier k % 2.
     auto wait_in = [&](int k) {
-        if (remote) mbar_wait_cluster(my_in + 8 * NW * (k & 1), (k >> 1) & 1, dead, a.fault);
-        else mbar_wait(my_in + 8 * NW * (k & 1), (k >> 1) & 1, dead, a.fault);
+        if (remote) mbar_wait_cluster(my_in + 8 * NW * (k & 1), (k >> 1) & 1, wait_words, a.fault);
+        else mbar_wait(my_in + 8 * NW * (k & 1), (k >> 1) & 1, wait_words, a.fault);
     };
     auto publish = [&](int k) {                      // the input of stage k is stored
         __syncwarp();
@@ -288,12 +266,12 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
         const double r = cta_total(slot);
         __syncwarp();
         mbar_arrive(bar_free + 8 * slot, lane == 0);
-        mbar_wait_cluster(bar_tfree + 8 * slot, phase ^ 1, dead, a.fault);
+        mbar_wait_cluster(bar_tfree + 8 * slot, phase ^ 1, wait_words, a.fault);
         if ((lane % span) == 0) flow_st_cluster(tot0 + 8u * ((slot * CS + rank) * NV + lane / span), r);
         __syncwarp();
         mbar_arrive_cluster(flow_map(bar_tot + 8 * slot, 0), lane == 0);
         if (rank != 0) return;
-        mbar_wait_cluster(bar_tot + 8 * slot, phase, dead, a.fault);
+        mbar_wait_cluster(bar_tot + 8 * slot, phase, wait_words, a.fault);
         write_row(slot, row);
         __syncwarp();
         mbar_arrive_cluster(flow_map(bar_tfree + 8 * slot, lane < CS ? lane : 0), lane < CS);
@@ -311,8 +289,10 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
     double part[NV];
     if (warp == ncw) {
         for (long long n = n0 + save_left; n < n1; n += a.save_every, ++row) {
-            mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, dead, a.fault);
+            mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
+            if (gave_up(wait_words)) break;
             finish_row(row % kFlowRows, row0 + row, (row / kFlowRows) & 1);
+            if (gave_up(wait_words)) break;
         }
     } else {
         publish(0);
@@ -321,13 +301,14 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
             save_left = observe ? a.save_every - 1 : save_left - 1;
             const bool driven = DRIVE && __any_sync(0xffffffffu, cur_f != 0.0);   // 0*d adds exactly 0
             double next_f = 0.0;
+            bool leave = false;
             if (stager && step + 1 < n1) next_f = dtab[(step + 1) * NE];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
                 const int rb = s & 1;                // buffer read in this stage; the other one is written
                 const int ti = s == 0 ? 0 : (s == 3 ? 2 : 1);
                 if (s == 1 && observe) {
-                    mbar_wait(bar_free + 8 * (row % kFlowRows), ((row / kFlowRows) & 1) ^ 1, dead, a.fault);
+                    mbar_wait(bar_free + 8 * (row % kFlowRows), ((row / kFlowRows) & 1) ^ 1, wait_words, a.fault);
                     store_partials(part, row % kFlowRows);
                 }
                 const double(&S)[NAT][3] = s == 0 ? y : yc;
@@ -368,12 +349,16 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
                     }
                 push_all(rb ^ 1, s == NS - 1 ? y : yc);
                 publish(s + 1);
+                if (s == NS - 2) leave = gave_up(wait_words);      // here, where the wait and the field sums hide it
             }
             cur_f = next_f;
             if (observe) ++row;
+            if (leave) break;
         }
     }
-    flow_cluster_sync();                             // every store into this CTA has landed, every row is written
+    // every store into this CTA has landed, every row is written; and where a wait gave up, no CTA leaves while others
+    // (whose own waits for it then run out) may still store into it
+    flow_cluster_sync();
     if (slice + 1 < a.slices) {
         if (own) write_state(a.y_mid + b * N3);
         return;

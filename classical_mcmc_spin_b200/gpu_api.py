@@ -88,6 +88,11 @@ class GPULatticeDataHandle:
         runs and uneven batches run each call's launches as one captured graph.  Off: direct launches."""
         check(nat.lib().cmd_set_graphs(self.ptr, int(bool(enable))), "cmd_set_graphs")
 
+    def set_wait_limit(self, ns: int) -> None:
+        """Limit of the waits between the warps of a resident run (2^30 ns unless set); a run whose wait exceeds it
+        ends with CMD_ERR_WATCHDOG."""
+        check(nat.lib().cmd_set_wait_limit(self.ptr, int(ns)), "cmd_set_wait_limit")
+
     def rk45_variants(self) -> list:
         """[(index, name, holds this lattice)] of the on-chip controlled Dormand-Prince tilings."""
         L = nat.lib()

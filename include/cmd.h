@@ -358,6 +358,16 @@ int cmd_autotune(cmd_handle* h, int64_t B, int64_t n_steps, int32_t* best, doubl
 int cmd_set_graphs(cmd_handle* h, int32_t enable);
 
 /*
+ * Resident RK4 and SSPRK53 kernels wait between the warps of a trajectory.  Every
+ * such wait is bounded: one that is not met within `ns` nanoseconds (2^30 unless
+ * set; a stage takes about 1000) makes the run skip its remaining steps and the
+ * call return CMD_ERR_WATCHDOG; the handle stays usable.  A limit of 0 gives up
+ * as soon as a wait has been tried a few thousand times.  No reference
+ * counterpart.
+ */
+int cmd_set_wait_limit(cmd_handle* h, int64_t ns);
+
+/*
  * Tilings of the on-chip controlled Dormand-Prince kernel (CMD_RK45 in
  * cmd_integrate and cmd_run_uneven): CTAs per trajectory (one CTA or a
  * thread-block cluster of 2..16) x threads per CTA x sites per thread, with y

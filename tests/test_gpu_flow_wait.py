@@ -1,0 +1,46 @@
+"""The bounded waits of the resident flow kernels: what a wait that gives up returns, and that a healthy run never
+does."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = ["rk4_flow<2,3,1> maxt=160", "rk4_cluster_flow<2,3,1> cs=2", "rk4_cluster_flow<2,3,1> cs=4"]
+
+
+@pytest.fixture(scope="module")
+def api(native):
+    from classical_mcmc_spin_b200 import gpu_api
+    return gpu_api
+
+
+def _handle(kernel):
+    """8x16 honeycomb (32 cells on each of four CTAs) pinned to a kernel, and its initial spins."""
+    from classical_mcmc_spin_b200.lattice import Lattice
+    from classical_mcmc_spin_b200.states import random_unit_spins
+    lat = Lattice.kitaev(8, 16, 1)
+    h = lat.to_gpu()
+    h.set_variant(next(i for i, name, fits in h.variants() if fits and name.startswith(kernel)))
+    return h, random_unit_spins(lat.lattice_size, 5).ravel()
+
+
+def _short_run(api, h, s0):
+    api.set_gpu_spins(h, s0)
+    _, obs, _ = api.integrate_gpu(h, 0.0, 0.395, 0.01, 3, "rk4", with_states=False)
+    return obs, api.get_gpu_spins(h)
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_a_wait_that_gives_up_returns_a_status_and_leaves_the_handle_usable(api, native, kernel):
+    """A limit of 0 ends the wait for a row 30000 steps away after a few thousand tries: the run skips its other steps
+    and returns CMD_ERR_WATCHDOG, every CTA of a cluster staying to the end; the next run is as before."""
+    h, s0 = _handle(kernel)
+    obs, fin = _short_run(api, h, s0)
+    h.set_wait_limit(0)
+    with pytest.raises(native.CmdError) as e:
+        api.integrate_gpu(h, 0.0, 299.9995, 0.001, 30000, "rk4", with_states=False)
+    assert e.value.code == native.CMD_ERR_WATCHDOG
+    h.set_wait_limit(1 << 30)
+    obs2, fin2 = _short_run(api, h, s0)
+    np.testing.assert_array_equal(obs2, obs)
+    np.testing.assert_array_equal(fin2, fin)
