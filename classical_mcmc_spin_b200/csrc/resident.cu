@@ -82,6 +82,7 @@ int launch_flow(const cmd_handle* h, const cmd::ResidentArgs& args, const double
     a.B = B;
     a.fault = h->hfault.as<int>();
     a.wait_ns = (unsigned long long)h->wait_ns;
+    a.row_ns = flow_row_ns(a.wait_ns, (unsigned long long)std::min<int64_t>(a.save_every, a.n_steps));
     if (h->lay.paired) a.nbr = h->nbrp.as<int>();
     // items are (slice, trajectory), trajectories fastest: the earlier slice of an item ran in an earlier launch
     // (slots <= B), so stream order is the only dependence
@@ -149,6 +150,7 @@ int launch_flow_cluster(const cmd_handle* h, const cmd::ResidentArgs& args, cons
     a.B = B;
     a.fault = h->hfault.as<int>();
     a.wait_ns = (unsigned long long)h->wait_ns;
+    a.row_ns = flow_row_ns(a.wait_ns, (unsigned long long)std::min<int64_t>(a.save_every, a.n_steps));
     FlowClusterArgs fc{};
     const Layout::FlowCluster& t = h->lay.flow_cluster[CS];
     fc.Gc = (int)cluster_cells(h->lay.G, CS);

@@ -70,13 +70,13 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar, bool on) {
         "@p mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"((unsigned)on) : "memory");
 }
 // Waits until the phase of `parity` of the mbarrier completes (acquire, at the named scope).  Bounded: a thread that
-// has tried kWaitTries times and for longer than FlowWait::ns (the tries too, so that time in which the GPU runs another
+// has tried kWaitTries times and for longer than its limit in FlowWait (the tries too, so that time in which the GPU runs another
 // process does not count) sets FlowWait::dead and *fault (host) and goes on, as does one that finds `dead` set; every
 // warp of the CTA looks at `dead` once a step and leaves the step loop (gave_up).  No thread ends early: a CTA of a
 // cluster stays while others may store into it, and every thread meets the barriers after the loop.  One block of
 // inline PTX: as a call, or as C++ after a failed first try, the cold path costs the hot one spills.
 constexpr unsigned kWaitTries = 4096;
-#define CMD_MBAR_WAIT(SCOPE)                                                                                 \
+#define CMD_MBAR_WAIT(SCOPE, LIMIT)                                                                          \
     asm volatile(                                                                                            \
         "{\n\t.reg .pred p;\n\t.reg .u64 t0, t1, lim;\n\t.reg .u32 d, n;\n\t"                               \
         "mbarrier.try_wait.parity.acquire." SCOPE ".shared::cta.b64 p, [%0], %1;\n\t"                        \
@@ -92,7 +92,7 @@ constexpr unsigned kWaitTries = 4096;
         "add.u32 n, n, 1;\n\t"                                                                               \
         "mov.u64 t1, %%globaltimer;\n\t"                                                                     \
         "sub.u64 t1, t1, t0;\n\t"                                                                            \
-        "ld.shared::cta.u64 lim, [%2+8];\n\t"                                                                \
+        "ld.shared::cta.u64 lim, [%2+%5];\n\t"                                                               \
         "setp.le.u64 p, t1, lim;\n\t"                                                                        \
         "@p bra AGAIN;\n\t"                                                                                  \
         "setp.lt.u32 p, n, %4;\n\t"                                                                          \
@@ -102,11 +102,15 @@ constexpr unsigned kWaitTries = 4096;
         "st.volatile.global.u32 [%3], d;\n"                                                                  \
         "DONE:\n\t}"                                                                                         \
         :                                                                                                    \
-        : "r"(bar), "r"(parity), "r"(words), "l"(fault), "n"(kWaitTries)                                     \
+        : "r"(bar), "r"(parity), "r"(words), "l"(fault), "n"(kWaitTries), "n"(LIMIT)                         \
         : "memory")
 
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t words, int* fault) {
-    CMD_MBAR_WAIT("cta");
+    CMD_MBAR_WAIT("cta", offsetof(FlowWait, ns));
+}
+// The helper warp's wait for a row, which is as many steps away as the caller saves rows apart.
+__device__ __forceinline__ void mbar_wait_row(uint32_t bar, uint32_t parity, uint32_t words, int* fault) {
+    CMD_MBAR_WAIT("cta", offsetof(FlowWait, row_ns));
 }
 // Whether a wait of the CTA gave up, the same answer in every lane of the warp.
 __device__ __forceinline__ bool gave_up(uint32_t words) {
@@ -157,7 +161,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     int pb[NAT][NL > 0 ? NL : 1];                    // word offset of each partner's component 0 in buffer 0
     const double* y0 = slice == 0 ? a.y0 + b * a.y0_stride : a.y_mid + b * N3;
     if (tid < 32) dep[tid] = 0;
-    flow_wait_init(fw, tid, a.wait_ns);
+    flow_wait_init(fw, tid, a.wait_ns, a.row_ns);
 #pragma unroll
     for (int at = 0; at < NAT; ++at)
 #pragma unroll
@@ -298,7 +302,7 @@ rk4_flow_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __grid_const
     double part[NV];
     if (HELP && warp == ncw) {
         for (long long n = n0 + save_left; n < n1; n += a.save_every, ++row) {
-            mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
+            mbar_wait_row(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
             if (gave_up(wait_words)) break;
             finish_row(row % kFlowRows, row0 + row);
         }

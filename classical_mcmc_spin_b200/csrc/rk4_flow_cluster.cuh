@@ -60,7 +60,7 @@ __device__ __forceinline__ void flow_cluster_sync() {
 
 // mbar_wait with cluster-scope acquire.
 __device__ __forceinline__ void mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t words, int* fault) {
-    CMD_MBAR_WAIT("cluster");
+    CMD_MBAR_WAIT("cluster", offsetof(FlowWait, ns));
 }
 
 template <int NAT, int Z, int LZ, int CS, int MAXT, bool STAT, bool DRIVE, bool PAIR>
@@ -144,7 +144,7 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
         mbar_init(bar_tot + 8 * tid, CS);
         mbar_init(bar_tfree + 8 * tid, 1);
     }
-    flow_wait_init(fw, tid, a.wait_ns);
+    flow_wait_init(fw, tid, a.wait_ns, a.row_ns);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     flow_cluster_sync();                             // every CTA's barriers exist
     const uint32_t my_in = bar_in + 8 * warp;
@@ -289,7 +289,7 @@ rk4_flow_cluster_kernel(const __grid_constant__ Couplings<NAT, Z> cp, const __gr
     double part[NV];
     if (warp == ncw) {
         for (long long n = n0 + save_left; n < n1; n += a.save_every, ++row) {
-            mbar_wait(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
+            mbar_wait_row(bar_full + 8 * (row % kFlowRows), (row / kFlowRows) & 1, wait_words, a.fault);
             if (gave_up(wait_words)) break;
             finish_row(row % kFlowRows, row0 + row, (row / kFlowRows) & 1);
             if (gave_up(wait_words)) break;

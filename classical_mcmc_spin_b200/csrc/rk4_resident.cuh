@@ -77,7 +77,7 @@ struct ResidentArgs {
     double* y_mid;            // [B][N*3] states between slices
     int method;               // host: CMD_RK4 or CMD_SSPRK53
     int* fault;               // set when a wait inside the kernel gave up (host-visible)
-    unsigned long long wait_ns;   // limit of a wait inside the kernel
+    unsigned long long wait_ns, row_ns;   // limits of the waits inside the kernel (FlowWait)
 };
 
 constexpr int kRedStride = 16;  // doubles per warp in the reduction scratch

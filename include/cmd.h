@@ -361,9 +361,10 @@ int cmd_set_graphs(cmd_handle* h, int32_t enable);
  * Resident RK4 and SSPRK53 kernels wait between the warps of a trajectory.  Every
  * such wait is bounded: one that is not met within `ns` nanoseconds (2^30 unless
  * set; a stage takes about 1000) makes the run skip its remaining steps and the
- * call return CMD_ERR_WATCHDOG; the handle stays usable.  A limit of 0 gives up
- * as soon as a wait has been tried a few thousand times.  No reference
- * counterpart.
+ * call return CMD_ERR_WATCHDOG; the handle stays usable.  The wait for the next
+ * observable row has this limit for every wait of the steps before it, so the
+ * save interval is not bounded.  A limit of 0 gives up as soon as a wait has
+ * been tried a few thousand times.  No reference counterpart.
  */
 int cmd_set_wait_limit(cmd_handle* h, int64_t ns);
 

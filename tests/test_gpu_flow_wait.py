@@ -44,3 +44,25 @@ def test_a_wait_that_gives_up_returns_a_status_and_leaves_the_handle_usable(api,
     obs2, fin2 = _short_run(api, h, s0)
     np.testing.assert_array_equal(obs2, obs)
     np.testing.assert_array_equal(fin2, fin)
+
+
+@pytest.mark.parametrize("kernel,limit,gap", [(k, 10**6, 30000) for k in KERNELS] +
+                         [(KERNELS[0], 1 << 30, 900000), (KERNELS[1], 1 << 30, 600000)])
+def test_rows_may_lie_further_apart_than_a_wait_may_last(api, kernel, limit, gap):
+    """The wait for a row lasts as many steps as the caller saves rows apart (57 ms at 30000 steps, over 1.1 s in the
+    last two): the run equals the same one in pieces of one gap, bit for bit."""
+    h, s0 = _handle(kernel)
+    dt = 1e-4
+    h.set_wait_limit(limit)
+    api.set_gpu_spins(h, s0)
+    _, obs, times = api.integrate_gpu(h, 0.0, (2 * gap - 0.5) * dt, dt, gap, "rk4", with_states=False)
+    fin = api.get_gpu_spins(h)
+    assert len(times) == 3
+    api.set_gpu_spins(h, s0)
+    rows = []
+    for piece in range(2):
+        _, o, _ = api.integrate_gpu(h, 0.0, (gap - 0.5) * dt, dt, gap // 10, "rk4", with_states=False)
+        rows += [o[0]] if piece == 0 else []
+        rows.append(o[-1])
+    np.testing.assert_array_equal(obs, np.stack(rows))
+    np.testing.assert_array_equal(fin, api.get_gpu_spins(h))
