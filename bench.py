@@ -325,6 +325,7 @@ def _forward_device(torch, dev, h, states, S, dt, streamed):
     run(S)
     e1.record(stream)
     torch.cuda.synchronize(dev)
+    h.run_status()
     ms = e0.elapsed_time(e1)
     value = B * N * S / (ms * 1e-3)
     out = {"value": value, "unit": UNIT, "ms": ms, "rk4_steps": S, "launches": launches.value,
@@ -635,6 +636,7 @@ def main():
         n_launch += launches.value
     t_end.record()
     torch.cuda.synchronize(dev)
+    h.run_status()
     clocks = sampler.stop()
     total_ms = t_start.elapsed_time(t_end)
     kern_ms = [a.elapsed_time(b) for a, b in ev]

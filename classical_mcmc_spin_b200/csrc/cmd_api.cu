@@ -1036,10 +1036,11 @@ int run_batch_chunked(cmd_handle* h, const cmd_batch_desc* d, const double* d_in
         if (done[i]) cudaEventDestroy(done[i]);
         if (copied[i]) cudaEventDestroy(copied[i]);
     }
+    const int fault = check_fault(h);                   // also cleared where something else failed
     if (rc != CMD_OK) return rc;
     if (e1 != cudaSuccess) return fail(CMD_ERR_CUDA, std::string("copy stream: ") + cudaGetErrorString(e1));
     if (e2 != cudaSuccess) return fail(CMD_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e2));
-    return CMD_OK;
+    return fault;
 }
 
 }  // namespace
@@ -1232,6 +1233,12 @@ int cmd_set_graphs(cmd_handle* h, int32_t enable) {
     h->graphs = enable != 0;
     if (!h->graphs) release_stream_graph(h);
     return CMD_OK;
+}
+
+int cmd_run_status(cmd_handle* h) {
+    cmd::clear_error();
+    if (int rc = check_handle(h, false)) return rc;
+    return check_fault(h);
 }
 
 int cmd_set_wait_limit(cmd_handle* h, int64_t ns) {

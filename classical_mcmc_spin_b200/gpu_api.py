@@ -93,6 +93,11 @@ class GPULatticeDataHandle:
         ends with CMD_ERR_WATCHDOG."""
         check(nat.lib().cmd_set_wait_limit(self.ptr, int(ns)), "cmd_set_wait_limit")
 
+    def run_status(self) -> None:
+        """Raises CmdError (CMD_ERR_WATCHDOG) when a kernel gave up a wait since that was last reported; for
+        asynchronous calls (cmd_run_batch_device), after their stream has been synchronised."""
+        check(nat.lib().cmd_run_status(self.ptr), "cmd_run_status")
+
     def rk45_variants(self) -> list:
         """[(index, name, holds this lattice)] of the on-chip controlled Dormand-Prince tilings."""
         L = nat.lib()

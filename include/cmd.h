@@ -196,7 +196,8 @@ int64_t cmd_batch_rows(int64_t n_steps, int64_t save_interval);
  * pulse4 are device pointers; d1/d2 stay host arrays (they become kernel
  * parameters).  The call is asynchronous on `stream` (a cudaStream_t, NULL =
  * the handle's stream).  `launches` (may be NULL) gets the number of kernels
- * launched.
+ * launched.  CMD_OK says that the work was enqueued: once the stream has been
+ * synchronised, cmd_run_status says whether a kernel gave up a wait.
  */
 int cmd_run_batch_device(cmd_handle* h, const cmd_batch_desc* d, void* stream, int32_t* launches);
 
@@ -227,6 +228,15 @@ int cmd_run_batch_device(cmd_handle* h, const cmd_batch_desc* d, void* stream, i
  * writes itself, so nothing carries over between calls.
  */
 int cmd_run_batch_device_noalloc(cmd_handle* h, const cmd_batch_desc* d, void* stream, int32_t* launches);
+
+/*
+ * CMD_ERR_WATCHDOG, once, when a kernel of h gave up a wait (cmd_set_wait_limit)
+ * since that was last reported: the results of the calls since then are not to
+ * be used.  Else CMD_OK.  For asynchronous calls, after their stream has been
+ * synchronised; a call that synchronises reports (and clears) it by itself, one
+ * left over from an earlier asynchronous call too.  Reads host memory only.
+ */
+int cmd_run_status(cmd_handle* h);
 
 /*
  * 2DCS analysis step (restates util/readers_new/reader_honeycomb.py:459-553,

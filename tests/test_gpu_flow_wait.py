@@ -66,3 +66,51 @@ def test_rows_may_lie_further_apart_than_a_wait_may_last(api, kernel, limit, gap
         rows.append(o[-1])
     np.testing.assert_array_equal(obs, np.stack(rows))
     np.testing.assert_array_equal(fin, api.get_gpu_spins(h))
+
+
+def _batch(api, native, h, s0, n_steps, save):
+    """cmd_run_batch_device of two trajectories on a stream of its own, synchronised; its status says it was enqueued."""
+    import ctypes as C
+    import torch
+    states = torch.from_numpy(np.stack([s0, s0])).cuda()
+    obs = torch.zeros((2, native.lib().cmd_batch_rows(n_steps, save), 10), dtype=torch.float64, device="cuda")
+    d = native.BatchDesc()
+    d.B, d.states, d.method, d.width, d.dt = 2, states.data_ptr(), native.CMD_RK4, 1.0, 1e-3
+    d.n_steps, d.save_interval, d.obs = n_steps, save, obs.data_ptr()
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    native.check(native.lib().cmd_run_batch_device(h.ptr, C.byref(d), C.c_void_p(st.cuda_stream), None), "batch")
+    st.synchronize()
+
+
+def test_a_long_host_batch_reports_a_wait_that_gave_up(api, native):
+    """Time chunks (4096 steps or more) synchronise by themselves."""
+    h, s0 = _handle(KERNELS[0])
+    st = np.stack([s0, s0])
+    good = api.run_batch(h, st, 5000, 1e-3, save_interval=500)
+    h.set_wait_limit(0)
+    with pytest.raises(native.CmdError) as e:
+        api.run_batch(h, st, 320000, 1e-3, save_interval=20000)
+    assert e.value.code == native.CMD_ERR_WATCHDOG
+    h.set_wait_limit(1 << 30)
+    for a, b in zip(api.run_batch(h, st, 5000, 1e-3, save_interval=500), good):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("entry", ["status", "get_spins", "integrate", "batch", "chunked", "observables"])
+def test_an_asynchronous_calls_fault_is_reported_once(api, native, entry):
+    h, s0 = _handle(KERNELS[0])
+    api.set_gpu_spins(h, s0)
+    call = {"status": h.run_status, "get_spins": lambda: api.get_gpu_spins(h), "observables": lambda: api.observables_gpu(h),
+            "integrate": lambda: api.integrate_gpu(h, 0.0, 0.095, 0.01, 5, "rk4", with_states=False),
+            "batch": lambda: api.run_batch(h, s0[None], 10, 0.01), "chunked": lambda: api.run_batch(h, s0[None], 4096, 0.01)}[entry]
+    call()
+    h.set_wait_limit(0)
+    _batch(api, native, h, s0, 60000, 20000)
+    h.set_wait_limit(1 << 30)
+    with pytest.raises(native.CmdError) as e:
+        call()
+    assert e.value.code == native.CMD_ERR_WATCHDOG
+    call()
+    _batch(api, native, h, s0, 100, 10)
+    h.run_status()
