@@ -39,6 +39,17 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// A table uploaded on first use: d holds memory only once its contents are there, so a copy that failed is made again
+// by the next call.
+inline int upload_once(DevBuf& d, const void* src, size_t bytes, const char* what) {
+    if (d.p) return CMD_OK;
+    if (int rc = d.ensure(bytes ? bytes : sizeof(int))) return rc;
+    const cudaError_t e = bytes ? cudaMemcpy(d.p, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+    if (e == cudaSuccess) return CMD_OK;
+    d.release();
+    return fail(CMD_ERR_CUDA, std::string(what) + " upload: " + cudaGetErrorString(e));
+}
+
 // Page-locked host buffer, grown on demand (device-to-host copies into it run
 // at full link speed and asynchronously).
 struct HostBuf {

@@ -267,6 +267,8 @@ int variant_count() { return kNumVariants; }
 // (atom*3)*G + cell become (rank << 24) | ((atom*3)*Gc + cell - rank*Gc) with
 // Gc = ceil(G / CS) cells per CTA.  Built once per handle.
 int upload_cluster_table(cmd_handle* h, int cs) {
+    DevBuf& d = cs == 2 ? h->cnbr2 : h->cnbr4;
+    if (d.p) return CMD_OK;
     const Layout& L = h->lay;
     const int64_t G = L.G, Gc = cluster_cells(G, cs);
     if ((int64_t)L.NA * 3 * Gc >= (1 << cmd::kClusterRankShift)) return CMD_OK;   // never launched
@@ -278,12 +280,7 @@ int upload_cluster_table(cmd_handle* h, int cs) {
         const int64_t r = gp / Gc, l = gp - r * Gc;
         t[i] = (int)((r << cmd::kClusterRankShift) | ((at * 3 + comp) * Gc + l));
     }
-    DevBuf& d = cs == 2 ? h->cnbr2 : h->cnbr4;
-    if (d.p) return CMD_OK;
-    if (int rc = d.ensure(std::max<size_t>(t.size(), 1) * sizeof(int))) return rc;
-    if (!t.empty() && cudaMemcpy(d.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
-        return fail(CMD_ERR_CUDA, "cluster neighbour table upload failed");
-    return CMD_OK;
+    return upload_once(d, t.data(), t.size() * sizeof(int), "cluster neighbour table");
 }
 
 // Partner words of the cluster layout with CS CTAs (CS = 1: the global offsets, rank 0).
@@ -351,9 +348,7 @@ int prepare_variant(cmd_handle* h, int vi) {
     std::vector<int> all(t.pw);
     all.insert(all.end(), t.push.begin(), t.push.end());
     all.insert(all.end(), t.peers.begin(), t.peers.end());
-    if (int rc = d.ensure(all.size() * sizeof(int))) return rc;
-    CUDA_TRY(cudaMemcpy(d.p, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice));
-    return CMD_OK;
+    return upload_once(d, all.data(), all.size() * sizeof(int), "cluster flow table");
 }
 
 bool variant_fits(const Variant& v, const Layout& L) {

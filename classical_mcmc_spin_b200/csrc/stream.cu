@@ -74,9 +74,7 @@ int stream_table(cmd_handle* h, bool pair) {
                 const int64_t off = src[((size_t)g * L.NA + a) * NL + m], at = off / (3 * L.G);
                 t[((size_t)a * NL + m) * L.G + g] = soff<NAT>((int)(off - at * 3 * L.G), (int)at);
             }
-    if (int rc = d.ensure(t.size() * sizeof(int))) return rc;
-    CUDA_TRY(cudaMemcpy(d.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice));
-    return CMD_OK;
+    return upload_once(d, t.data(), t.size() * sizeof(int), "streamed partner table");
 }
 
 // One launch of RK stage s.
