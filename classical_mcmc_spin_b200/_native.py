@@ -112,6 +112,7 @@ _SIGS = {
     "cmd_variant_info": (C.c_int, [C.c_void_p, C.c_int32, C.c_char_p, C.c_int32, _I32]),
     "cmd_set_variant": (C.c_int, [C.c_void_p, C.c_int32]),
     "cmd_get_variant": (C.c_int, [C.c_void_p, _I32]),
+    "cmd_batch_variant": (C.c_int, [C.c_void_p, C.c_int64, C.c_int32, _I32]),
     "cmd_autotune": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, _I32, _D]),
     "cmd_set_graphs": (C.c_int, [C.c_void_p, C.c_int32]),
     "cmd_set_wait_limit": (C.c_int, [C.c_void_p, C.c_int64]),

@@ -424,9 +424,8 @@ int cmd_create(const cmd_lattice_desc* d, cmd_handle** out) {
                                            cudaMemcpyHostToDevice) != cudaSuccess)
                 rc = fail(CMD_ERR_CUDA, "neighbour table upload failed");
         }
-        // the table of the default variant's clusters; the others when a variant or the adjoint first needs them
-        const int vi = default_variant(h->lay);
-        if (rc == CMD_OK && vi >= 0) rc = prepare_variant(h, vi);
+        // the cluster tables that batches may need; those of a pinned variant or of the adjoint on their first use
+        if (rc == CMD_OK) rc = prepare_defaults(h);
     }
     if (rc == CMD_OK) *h->hfault.as<int>() = 0;
     if (rc == CMD_OK) rc = h->state.ensure((size_t)h->N * 3 * sizeof(double));
@@ -1175,6 +1174,14 @@ int cmd_get_variant(cmd_handle* h, int32_t* idx) {
     if (int rc = check_handle(h, false)) return rc;
     if (!idx) return fail(CMD_ERR_INVALID_ARG, "NULL output");
     *idx = pick_variant(h);
+    return CMD_OK;
+}
+
+int cmd_batch_variant(cmd_handle* h, int64_t B, int32_t driven, int32_t* idx) {
+    cmd::clear_error();
+    if (int rc = check_handle(h, false)) return rc;
+    if (!idx || B <= 0) return fail(CMD_ERR_INVALID_ARG, "NULL output or bad batch size");
+    *idx = batch_variant(h, B, driven != 0);
     return CMD_OK;
 }
 

@@ -258,7 +258,9 @@ bool variant_fits(const Variant& v, const Layout& L);
 int default_variant(const Layout& L);
 // Uploads the tables variant vi reads (synchronous, once per handle).
 int prepare_variant(cmd_handle* h, int vi);
+int prepare_defaults(cmd_handle* h);
 int pick_variant(const cmd_handle* h);
+int batch_variant(const cmd_handle* h, int64_t B, bool drive);
 int flow_variant(const Layout& L);
 bool stages_room(cmd_handle* h, int64_t n_steps);
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches);

@@ -63,7 +63,7 @@ constexpr int64_t noalloc_round(int64_t n) { return (n + 31) / 32 * 32; }   // 2
 // table, raw rows), so nothing needs clearing between calls.
 int run_resident_noalloc(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches) {
     int32_t nl = 0;
-    const int vi = pick_variant(h);
+    const int vi = batch_variant(h, r.B, r.pulses && r.n_steps > 0);
     if (vi < 0 || !variant_fits(variant_table()[vi], h->lay)) {
         if (!h->lay.uniform) return no_instance(h->lay);
         return fail(CMD_ERR_UNSUPPORTED, "cmd_run_batch_device_noalloc runs resident lattices only (one CTA or a "

@@ -428,11 +428,21 @@ int64_t resident_launches(const ResidentArgs& a, int64_t B) {
     return a.slices > 1 ? (B * a.slices + a.slots - 1) / a.slots : 1;
 }
 
+// The cluster flow kernel that batch_variant may choose in place of default variant vi, or -1.
+static int cluster_alternative(const Layout& L, int vi) {
+    if (vi < 0 || kVariants[vi].CS > 1 || kVariants[vi].flow) return -1;
+    for (int i = 0; i < kNumVariants; ++i)
+        if (kVariants[i].flow && kVariants[i].CS > 1 && variant_fits(kVariants[i], L)) return i;
+    return -1;
+}
+
 // The variant of a batch of B trajectories: the handle's, but where nothing was pinned and the default is a
 // one-CTA kernel with a stage barrier, the cluster flow kernel if every trajectory's cluster is resident at once (SMs
 // would idle otherwise), or always where that CTA would hold two 4-atom cells per thread.  B200, per stage and
 // trajectory, one CTA against clusters of 2: honeycomb 27x31 1.63 us on one SM, 0.94 us on two; pyrochlore 500 cells
-// 2.47 / 1.93 us, 864 cells (two per thread, spills) 8.66 / 2.84 us.
+// 2.47 / 1.93 us, 864 cells (two per thread, spills) 8.66 / 2.84 us.  The line does not count what slices give the
+// clusters of a larger batch: by these figures they would lead a little further (to about 1.7 waves of clusters).
+// The two kernels add in different orders, so a trajectory's last bits depend on B there (cmd_batch_variant).
 int batch_variant(const cmd_handle* h, int64_t B, bool drive) {
     const int vi = pick_variant(h);
     if (vi < 0 || vi == h->variant || kVariants[vi].CS > 1) return vi;
@@ -445,12 +455,18 @@ int batch_variant(const cmd_handle* h, int64_t B, bool drive) {
         }
         return vi;
     }
-    for (int i = 0; i < kNumVariants; ++i) {
-        const Variant& v = kVariants[i];
-        if (!v.flow || v.CS == 1 || !variant_fits(v, h->lay)) continue;
-        return (kVariants[vi].NAT == 4 && kVariants[vi].CPT > 1) || B <= v.slots(h, drive) ? i : vi;
-    }
-    return vi;
+    const int alt = cluster_alternative(h->lay, vi);
+    if (alt < 0) return vi;
+    return (kVariants[vi].NAT == 4 && kVariants[vi].CPT > 1) || B <= kVariants[alt].slots(h, drive) ? alt : vi;
+}
+
+// Uploads the tables of every variant that batches of h may run without a pin.
+int prepare_defaults(cmd_handle* h) {
+    const int vi = default_variant(h->lay);
+    if (vi < 0) return CMD_OK;
+    if (int rc = prepare_variant(h, vi)) return rc;
+    const int alt = cluster_alternative(h->lay, vi);
+    return alt >= 0 ? prepare_variant(h, alt) : CMD_OK;
 }
 
 // Room for the envelope table of n_steps driven SSPRK53 steps.

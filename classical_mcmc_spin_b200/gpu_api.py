@@ -75,6 +75,12 @@ class GPULatticeDataHandle:
         check(nat.lib().cmd_get_variant(self.ptr, C.byref(v)), "cmd_get_variant")
         return v.value
 
+    def batch_variant(self, B: int, driven: bool = False) -> int:
+        """Variant that a batch of B trajectories runs (the pinned one, else by lattice and B)."""
+        v = C.c_int32()
+        check(nat.lib().cmd_batch_variant(self.ptr, int(B), int(bool(driven)), C.byref(v)), "cmd_batch_variant")
+        return v.value
+
     def autotune(self, B: int, n_steps: int) -> tuple:
         """Times every fitting variant; pins and returns (best index, ms per variant)."""
         n = nat.lib().cmd_variant_count()

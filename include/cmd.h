@@ -256,7 +256,8 @@ int cmd_nonlinear_spectrum(const double* M0, const double* M1, const double* M01
  * info[0] = sites per group (unit-cell atoms), info[1] = groups,
  * info[2] = max bonds per site kept, info[3] = threads per block of the
  * resident RK4 kernel that hold groups, info[4] = groups per thread, info[5] =
- * shared-memory bytes per trajectory (cluster kernels: of a CTA's own groups). */
+ * shared-memory bytes per trajectory (cluster kernels: of a CTA's own groups).
+ * Of the pinned or default variant; a batch may run another (cmd_batch_variant). */
 int cmd_layout_info(cmd_handle* h, int64_t* info);
 
 /*
@@ -336,7 +337,17 @@ int cmd_adjoint_rk4(cmd_handle* h, const cmd_adjoint_desc* d);
  *   cmd_variant_count     number of variants in the library
  *   cmd_variant_info      name of variant idx and whether it fits h's lattice
  *   cmd_set_variant       pin a variant for h (-1: back to the default choice)
- *   cmd_get_variant       variant h uses now
+ *   cmd_get_variant       the pinned or tuned variant, else the lattice's default
+ *                         (-1: streamed stages)
+ *   cmd_batch_variant     variant a batch of B trajectories runs, with or without
+ *                         a drive.  The pinned or tuned one; without a pin the
+ *                         default, except that lattices of 641 to 1024 2-atom or
+ *                         257 to 512 4-atom cells run a batch on the cluster
+ *                         kernel when all of its clusters fit the GPU at once
+ *                         (and on one CTA each when they do not).  The two kernels
+ *                         add in different orders, so for those lattices the last
+ *                         bits of a trajectory depend on the batch it is run in;
+ *                         pin a variant where they must not
  *   cmd_autotune          time every fitting variant on a B-trajectory,
  *                         n_steps-step batch from h's current spins, pin the
  *                         fastest; ms[cmd_variant_count()] gets the times
@@ -346,6 +357,7 @@ int cmd_variant_count(void);
 int cmd_variant_info(cmd_handle* h, int32_t idx, char* name, int32_t name_len, int32_t* fits);
 int cmd_set_variant(cmd_handle* h, int32_t idx);
 int cmd_get_variant(cmd_handle* h, int32_t* idx);
+int cmd_batch_variant(cmd_handle* h, int64_t B, int32_t driven, int32_t* idx);
 int cmd_autotune(cmd_handle* h, int64_t B, int64_t n_steps, int32_t* best, double* ms);
 
 /*
