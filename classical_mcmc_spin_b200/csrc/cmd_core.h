@@ -266,6 +266,7 @@ bool stages_room(cmd_handle* h, int64_t n_steps);
 int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* launches);
 // Sets a.slices / a.slots of a resident batch (a.drive set); the caller provides a.y_mid when a.slices > 1.
 void plan_slices(const cmd_handle* h, const Variant& V, int64_t B, int64_t n_steps, ResidentArgs& a);
+bool may_slice(const RunSpec& r, int64_t n3);
 int64_t resident_launches(const ResidentArgs& a, int64_t B);
 int upload_cluster_table(cmd_handle* h, int cs);
 const int* cluster_table(const cmd_handle* h, int cs);

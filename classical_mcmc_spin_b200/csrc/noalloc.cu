@@ -132,8 +132,7 @@ int run_resident_noalloc(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32
     }
     // slices keep their states in the caller's final_states: without them the run is not sliced
     a.slices = 1;
-    const bool over = r.y0_stride == 0 && r.y0 >= r.y_out && r.y0 < r.y_out + r.B * h->N * 3;   // read by every start
-    if (r.y_out && !over) plan_slices(h, V, r.B, r.n_steps, a);
+    if (may_slice(r, h->N * 3)) plan_slices(h, V, r.B, r.n_steps, a);
     a.y_mid = r.y_out;
     static const double zeros[3 * 64] = {};
     if (int rc = V.fn(h, a, r.d1 ? r.d1 : zeros, r.d2 ? r.d2 : zeros, r.B, st)) return rc;

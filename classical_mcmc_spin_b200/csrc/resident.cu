@@ -424,6 +424,13 @@ void plan_slices(const cmd_handle* h, const Variant& V, int64_t B, int64_t n_ste
     if (cost(best) * 50 < cost(1) * 49) a.slices = best;
 }
 
+// Slices need the final states' memory, and that memory must not hold the one initial state that every trajectory's
+// first slice reads.
+bool may_slice(const RunSpec& r, int64_t n3) {
+    if (!r.y_out) return false;
+    return r.y0_stride != 0 || r.y0 + n3 <= r.y_out || r.y_out + r.B * n3 <= r.y0;
+}
+
 int64_t resident_launches(const ResidentArgs& a, int64_t B) {
     return a.slices > 1 ? (B * a.slices + a.slots - 1) / a.slots : 1;
 }
@@ -532,10 +539,9 @@ int run_resident(cmd_handle* h, const RunSpec& r, cudaStream_t st, int32_t* laun
     }
     if (r.obs && V.NAT != 2 && V.NAT != 4) return fail(CMD_ERR_UNSUPPORTED, "no row finisher for this cell size");
     // slices keep their states in the caller's final states (nothing of the handle's: calls without a drive may
-    // overlap on several streams); one shared initial state that those overwrite is read by every trajectory's start
-    const bool over = r.y0_stride == 0 && r.y_out && r.y0 >= r.y_out && r.y0 < r.y_out + r.B * h->N * 3;
+    // overlap on several streams)
     a.slices = 1;
-    if (r.y_out && !over) plan_slices(h, V, r.B, r.n_steps, a);
+    if (may_slice(r, h->N * 3)) plan_slices(h, V, r.B, r.n_steps, a);
     a.y_mid = r.y_out;
     static const std::vector<double> zeros(3 * 64, 0.0);
     const double* d1 = r.d1 ? r.d1 : zeros.data();
