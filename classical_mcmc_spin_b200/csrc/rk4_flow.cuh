@@ -24,14 +24,17 @@
 //     constant-bank operand without a branch per atom.
 // Waits are bounded (mbar_wait); a run whose wait gave up skips its remaining steps and reports CMD_ERR_WATCHDOG.
 //
-// Bound: issue slots and the FP64 pipe.  24x24 honeycomb, one step's observables every step: 182 warp instructions
-// per warp and stage, 82 of them FP64; 18 warps put 5 on two of the SM's four schedulers, so the pipe needs 820 and
-// the issue port 910 of the stage's 1330 cycles there (0.68 us; 0.88 us with a CTA barrier per stage and 205
-// instructions).  B200, 1965 MHz: 768 driven trajectories x 2000 steps 32.1 ms (45.5 ms with the barrier and whole
-// waves; 36.9 ms with whole waves); one trajectory 2.80 us per step (3.61); 40 trajectories of 8x8 x 500 steps
-// 0.95 ms (1.35); 200 of the 1024-spin pyrochlore x 800 driven steps 4.35 ms (11.6 with the atoms in sequence; 5.27
-// without paired bonds); one 24x24 SSPRK53 trajectory x 400 steps, 11 states saved, 1.59 ms (7.05 in global memory,
-// where every RK vector is read and written each stage).  Polling progress words instead of waiting on mbarriers: 256 instructions, 0.83 us.
+// Bound: issue slots and the FP64 pipe.  24x24 honeycomb, one step's observables every step: 183 warp instructions
+// per warp and stage, 82 of them FP64 (209 and 92 with the drive); 18 warps put 5 on two of the SM's four schedulers,
+// so the pipe needs 820 and the issue port 915 of the stage's 1330 cycles there (0.68 us; 0.88 us with a CTA barrier
+// per stage and 205 instructions).  B200, 1965 MHz: 768 driven trajectories x 2000 steps 31.7 ms (45.5 ms with the
+// barrier and whole waves); one trajectory 2.78 us per step (3.61); 40 trajectories of 8x8 x 500 steps 0.94 ms (1.35);
+// 200 of the 1024-spin pyrochlore x 800 driven steps 4.26 ms (11.6 with the atoms in sequence); one 24x24 SSPRK53
+// trajectory x 400 steps, 11 states saved, 1.60 ms (7.05 in global memory, where every RK vector is read and written
+// each stage).  Polling progress words instead of waiting on mbarriers: 256 instructions, 0.83 us.  The look at
+// FlowWait::dead once a step stands after the publish of the last but one stage: 31.7 ms (32.1 with a flag in a
+// register that only the cold path sets and a vote, 31.9 in the middle of the last stage); lone undriven warps lose
+// 1-5 % to it.
 #pragma once
 
 #include "flow_wait.h"

@@ -11,9 +11,10 @@
 // pays a cluster barrier (~490 cycles) per stage in every warp, and a remote load per
 // component of a remote partner.
 //
-// B200, 48x48 honeycomb on 4 CTAs: 0.86 us a stage (1.54 with a cluster barrier per stage, 0.68
-// for one 24x24 CTA of the same size); 64 trajectories x 1000 steps 6.79 ms, sliced (11.98).
-// Pyrochlore, 1372 cells: 2.7 us a stage against 4.2.
+// B200, 48x48 honeycomb on 4 CTAs: 0.87 us a stage (1.54 with a cluster barrier per stage, 0.68
+// for one 24x24 CTA of the same size); 198 warp instructions per warp and stage, 82 of them FP64;
+// 64 trajectories x 1000 steps 6.91 ms, sliced (11.98; 6.81 without the look at FlowWait::dead once
+// a step, 7.03 with it in the middle of a stage).  Pyrochlore, 1372 cells: 2.7 us a stage against 4.2.
 //
 // Rows: each CTA's helper warp sums its warps' partials and stores them in CTA 0's totals
 // ring; CTA 0's helper adds them in rank order and writes the raw row.

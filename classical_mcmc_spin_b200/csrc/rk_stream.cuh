@@ -21,10 +21,10 @@
 //
 // Bound: latency of a short-lived CTA (partner offset, partner spins, store: two dependent
 // trips to L2) at 32 warps an SM; DRAM carries little once a group of trajectories fits L2.
-// B200, 65536-spin pyrochlore: 32 trajectories x 300 steps 46.0 ms (70.8 with rows of G cells,
-// one launch group, cell-major offsets and one kernel for all stages) = 5.6 TB/s of those
+// B200, 65536-spin pyrochlore: 32 trajectories x 300 steps 46.7-47.4 ms (70.8 with rows of G cells,
+// one launch group, cell-major offsets and one kernel for all stages) = 5.4-5.5 TB/s of those
 // 408 B; groups of a share of L2: 0.3 75.6, 0.4 69.3, 0.55-0.7 64.4, 0.9 68.4, all at once
-// 70.0 ms (before the blocked layout).  Adjoint of 8 x 100 steps 23.9 ms (34.3: a cell per
+// 70.0 ms (before the blocked layout).  Adjoint of 8 x 100 steps 24.1 ms (34.3: a cell per
 // thread, each partner's Hbar formed per bond from three vectors, couplings indexed at run
 // time); a VJP stage takes about 36 us.
 //
@@ -41,7 +41,7 @@
 
 namespace cmd {
 
-constexpr int kStreamTile = 256;     // cells per CTA (one cell per thread)
+constexpr int kStreamTile = 256;     // threads of a CTA (one site each)
 constexpr int kPart = 16;            // doubles per partial slot
 
 struct SVec {
@@ -52,7 +52,7 @@ struct SVec {
 
 struct StreamArgs {
     int G;                           // cells per trajectory
-    int tiles;                       // ceil(G / kStreamTile)
+    int tiles;                       // ceil(G / stream_cells<NAT>())
     int B;
     const int* nbr;                  // [NAT][Z-LZ][G] partner offsets, cell-minor: a warp's loads are consecutive
     double dt;

@@ -89,7 +89,7 @@ void stage(int s, dim3 grid, cudaStream_t st, const Couplings<NAT, Z>& cp, const
 }
 
 // Trajectories per group of a streamed run with `vectors` vectors of V doubles each: as many as keep the group's
-// vectors within kL2Share of L2 (measured on the 65536-spin pyrochlore, 32 trajectories: see rk_stream.cuh), in
+// vectors within kL2Share of L2 (measured on the 65536-spin pyrochlore, 32 trajectories, before the blocked layout: see rk_stream.cuh), in
 // groups of equal size.
 int64_t stream_group(const cmd_handle* h, int64_t B, int64_t V, int vectors) {
     int l2 = 0;
