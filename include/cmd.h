@@ -341,13 +341,14 @@ int cmd_adjoint_rk4(cmd_handle* h, const cmd_adjoint_desc* d);
  *                         (-1: streamed stages)
  *   cmd_batch_variant     variant a batch of B trajectories runs, with or without
  *                         a drive.  The pinned or tuned one; without a pin the
- *                         default, except that lattices of 641 to 1024 2-atom or
- *                         257 to 512 4-atom cells run a batch on the cluster
- *                         kernel when all of its clusters fit the GPU at once
- *                         (and on one CTA each when they do not).  The two kernels
- *                         add in different orders, so for those lattices the last
- *                         bits of a trajectory depend on the batch it is run in;
- *                         pin a variant where they must not
+ *                         default, except that lattices of 513 to 1024 4-atom
+ *                         cells run on the cluster kernel, and lattices of 641 to
+ *                         1024 2-atom or 257 to 512 4-atom cells do when all
+ *                         clusters of the batch fit the GPU at once (on one CTA
+ *                         each when they do not).  The two kernels add in
+ *                         different orders, so for the latter the last bits of a
+ *                         trajectory depend on the batch it is run in; pin a
+ *                         variant where they must not
  *   cmd_autotune          time every fitting variant on a B-trajectory,
  *                         n_steps-step batch from h's current spins, pin the
  *                         fastest; ms[cmd_variant_count()] gets the times
